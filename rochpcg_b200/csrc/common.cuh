@@ -151,8 +151,8 @@ inline cudaError_t launch_pdl_net(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
 // for the persistent kernels whose blocks meet at grid barriers.  Valid in
 // stream capture (the graph's kernel node keeps the attribute).
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_coop(void (*kernel)(KArgs...), unsigned grid, unsigned block, cudaStream_t s,
-                               Args&&... args)
+inline cudaError_t launch_coop_smem(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem,
+                                    cudaStream_t s, Args&&... args)
 {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -160,11 +160,18 @@ inline cudaError_t launch_coop(void (*kernel)(KArgs...), unsigned grid, unsigned
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_coop(void (*kernel)(KArgs...), unsigned grid, unsigned block, cudaStream_t s,
+                               Args&&... args)
+{
+    return launch_coop_smem(kernel, grid, block, 0, s, std::forward<Args>(args)...);
 }
 
 // Blocks of `kernel` that fit on the device at once (SMs x resident blocks

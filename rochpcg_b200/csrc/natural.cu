@@ -22,33 +22,11 @@ __global__ void __launch_bounds__(kNatBS) k_nat_spmv(NaturalLevel L, const doubl
     y[row] = sum;
 }
 
-// floor(a / 4) for any sign of a.
-__device__ __forceinline__ int floor_div4(int a) { return a >= 0 ? a / 4 : -((3 - a) / 4); }
-
-// One wavefront t of the Gauss-Seidel sweep (src/ComputeSYMGS_ref.cpp:68-85
-// for one row).  Thread (iy, j) takes iz = izmin + j, ix = t - 2 iy - 4 iz;
-// at most ceil(nx/4) + 1 values of iz meet 0 <= ix < nx for one (t, iy).
+// One wavefront t of the Gauss-Seidel sweep.
 __global__ void __launch_bounds__(kNatBS) k_nat_gs_front(NaturalLevel L, int t, int width,
                                                          const double* __restrict__ r, double* x)
 {
-    const int idx = blockIdx.x * kNatBS + threadIdx.x;
-    const int iy = idx / width;
-    const int j = idx - iy * width;
-    if(iy >= L.ny) return;
-    const int u = t - 2 * iy;  // ix + 4 iz
-    if(u < 0) return;
-    const int izmin = max(0, -floor_div4(L.nx - 1 - u));  // ceil((u - nx + 1) / 4)
-    const int iz = izmin + j;
-    if(iz >= L.nz || 4 * iz > u) return;
-    const int ix = u - 4 * iz;
-    const long long row = ((long long)iz * L.ny + iy) * L.nx + ix;
-    const size_t base = (size_t)row * kWidth;
-    const int n = L.nnz[row];
-    double sum = r[row];
-    for(int q = 0; q < n; ++q) sum = __dsub_rn(sum, __dmul_rn(L.val[base + q], x[L.ind[base + q]]));
-    const double d = L.val[base + L.diag_slot[row]];
-    sum = __dadd_rn(sum, __dmul_rn(x[row], d));  // remove the diagonal term of the loop
-    x[row] = __ddiv_rn(sum, d);
+    natural_front_row(L, t, width, blockIdx.x * kNatBS + threadIdx.x, r, x);
 }
 
 __global__ void k_nat_restrict(int nc, const int* __restrict__ f2c, const double* __restrict__ rf,
@@ -162,7 +140,7 @@ int launch_nat_spmv(const NaturalLevel& L, const double* x, double* y, cudaStrea
 int launch_nat_symgs(const NaturalLevel& L, const double* r, double* x, cudaStream_t s)
 {
     const int fronts = natural_fronts(L.nx, L.ny, L.nz);
-    const int width = (L.nx + 3) / 4 + 1;
+    const int width = natural_front_width(L.nx);
     const unsigned grid = grid_of((long long)L.ny * width, kNatBS);
     for(int t = 0; t < fronts; ++t)
     {

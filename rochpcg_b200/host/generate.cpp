@@ -273,6 +273,7 @@ void DeleteMatrix(SparseMatrix& A)
     dfree(A.d_matrixDiagonal);
     dfree(A.d_localToGlobalMap);
     dfree(A.d_rowHash);
+    dfree(A.referenceData);
     dfree(A.ell_col_ind);
     dfree(A.ell_val);
     dfree(A.diag_idx);
@@ -287,6 +288,7 @@ void DeleteMatrix(SparseMatrix& A)
     A.d_matrixDiagonal = nullptr;
     A.d_localToGlobalMap = nullptr;
     A.d_rowHash = nullptr;
+    A.referenceData = nullptr;
     A.ell_col_ind = nullptr;
     A.ell_val = nullptr;
     A.diag_idx = nullptr;

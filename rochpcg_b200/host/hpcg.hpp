@@ -89,6 +89,7 @@ struct SparseMatrix_STRUCT
     local_int_t* d_matrixDiagonal;
     global_int_t* d_localToGlobalMap;
     local_int_t* d_rowHash;
+    mutable void* referenceData;       // device workspace of ComputeSYMGS_ref, lives as long as the arrays above
 
     // ELL (src/SparseMatrix.hpp:131-141)
     local_int_t ell_width;

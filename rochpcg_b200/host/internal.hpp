@@ -71,6 +71,7 @@ struct Runtime
     hb::ReduceScratch* ws = nullptr;   // reduction scratch (ticket left at zero)
     double* d_scalar = nullptr;        // device result slots
     double* h_scalar = nullptr;        // pinned mirror
+    int* ref_status = nullptr;         // set by a reference sweep whose bounded wait ran out (device word)
 };
 Runtime& rt();
 void ensure_runtime();
@@ -190,6 +191,10 @@ inline const hb::ZgGroups* zg_of(const SparseMatrix& A)
     return o && o->zg_ok ? o->zg : nullptr;
 }
 inline MGOpt* mgopt(const SparseMatrix& A) { return A.mgData ? static_cast<MGOpt*>(A.mgData->optimizationData) : nullptr; }
+
+// HPCGB200_ERR_DEVICE_STATUS if a reference sweep's wait ran out since the
+// last check (synchronises the stream), defined in reference.cpp.
+int reference_status();
 
 // Operators on raw FP32 level data (mixed V-cycle), defined in operators.cpp.
 // pro: where this level's final values are prolongated (the finer level's x),

@@ -109,6 +109,8 @@ static void free_generated(SparseMatrix& A)
     dfree(A.d_mtxIndL);
     dfree(A.d_matrixValues);
     dfree(A.d_rowHash);
+    dfree(A.referenceData);
+    A.referenceData = nullptr;
     A.d_mtxIndL = nullptr;
     A.d_matrixValues = nullptr;
     A.d_rowHash = nullptr;

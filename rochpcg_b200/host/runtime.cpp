@@ -45,6 +45,8 @@ void ensure_runtime()
     g_rt.ws = static_cast<hb::ReduceScratch*>(p);
     HB_HOST_CUDA(cudaMalloc(&g_rt.d_scalar, 16 * sizeof(double)));
     HB_HOST_CUDA(cudaMallocHost(&g_rt.h_scalar, 16 * sizeof(double)));
+    HB_HOST_CUDA(cudaMalloc(&g_rt.ref_status, sizeof(int)));
+    HB_HOST_CUDA(cudaMemset(g_rt.ref_status, 0, sizeof(int)));
     g_rt.initialized = true;
 }
 
@@ -110,6 +112,7 @@ int HPCG_B200_Finalize()
     cudaStreamSynchronize(g_rt.stream);
     dfree(g_rt.ws);
     dfree(g_rt.d_scalar);
+    dfree(g_rt.ref_status);
     if(g_rt.h_scalar) cudaFreeHost(g_rt.h_scalar);
     g_rt = Runtime{};
     return 0;
