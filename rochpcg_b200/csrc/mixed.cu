@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "mixed.cuh"
+#include "small_level.cuh"
 #include "tma.cuh"
 
 namespace hb {
@@ -2148,6 +2149,8 @@ static cudaError_t pass_tma(const StencilLevel& L, const ColorLaunch& c, const S
 int launch32_symgs_zero(const StencilLevel& L, const float* diag32, const float* inv_diag32, const double* r64,
                         float* r32, float* x, cudaStream_t s, Prolong<float> pro)
 {
+    if(small_level_ok<float>(L, false))
+        return launch_small_zero<float>(L, diag32, inv_diag32, r64, r32, x, nullptr, nullptr, nullptr, s, pro);
     const int n = L.ncolors;
     const dim3 t(32, 8), t4(kV4X, kV4Y);
     const bool vec = vec4_ok(L);
@@ -2212,6 +2215,7 @@ int launch32_symgs_zero(const StencilLevel& L, const float* diag32, const float*
 int launch32_symgs(const StencilLevel& L, const float* inv_diag32, const float* r, float* x, double* z64,
                    cudaStream_t s, Prolong<float> pro)
 {
+    if(small_level_ok<float>(L, false)) return launch_small_symgs<float>(L, inv_diag32, r, x, z64, nullptr, s, pro);
     const int n = L.ncolors;
     const bool vec = vec4_ok(L);
     const bool tma = pass_tma_ok(L, x, pro);

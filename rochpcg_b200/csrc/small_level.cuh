@@ -1,0 +1,28 @@
+// SymGS steps of a small multigrid level as one cluster kernel (see
+// small_level.cu): the colour passes of launch32_symgs_zero / launch32_symgs
+// (FP32), launch64v_* (FP64 on the implicit stencil) and launch_symgs_zero /
+// launch_symgs (FP64 ELL values), bit for bit.
+#pragma once
+
+#include "mixed.cuh"
+
+namespace hb {
+
+// The level is small enough, canonically coloured and fits the cluster's
+// shared memory.  T: float, or double (ell: with the ELL values).
+template <typename T>
+bool small_level_ok(const StencilLevel& L, bool ell);
+
+// One zero-guess step: x from r; r64 (float only, may be null): r comes in
+// FP64 and its float copy is stored in r.  ell_val: the level's ELL values
+// (double only; null: the stencil's -1).  rc (may be null): also the residual
+// at the injected rows, rc[inj_c[i]] for row i of the parity-0 colour.
+template <typename T>
+int launch_small_zero(const StencilLevel& L, const T* diag, const T* inv_diag, const double* r64, T* r, T* x,
+                      const double* ell_val, const int* inj_c, T* rc, cudaStream_t s, Prolong<T> pro);
+// One full step on x.  z64 (float only, may be null): also the FP64 copy.
+template <typename T>
+int launch_small_symgs(const StencilLevel& L, const T* inv_diag, const T* r, T* x, double* z64,
+                       const double* ell_val, cudaStream_t s, Prolong<T> pro);
+
+}  // namespace hb

@@ -14,6 +14,7 @@
 #include "../csrc/learned.cuh"
 #include "../csrc/mixed.cuh"
 #include "../csrc/ops64.cuh"
+#include "../csrc/small_level.cuh"
 #include "hpcg.hpp"
 
 namespace hpcg_b200 {

@@ -35,24 +35,68 @@ int ComputeSPMV(const SparseMatrix& A, Vector& x, Vector& y)
     });
 }
 
+namespace {
+
+// The level runs its SymGS as one cluster kernel (small_level.cu): with T's
+// arithmetic, ell: on the ELL values.
+template <typename T>
+bool small_level(const SparseMatrix& A, bool ell)
+{
+    const LevelOpt* o = opt(A);
+    return o && o->stencil_ok && hb::small_level_ok<T>(o->st, ell);
+}
+
+// A small level's zero-guess step and, where it has a coarse grid, the
+// restriction of its residual to rc, in one kernel.
+int small_zero_restrict(const SparseMatrix& A, const double* r, double* x, const double* ell_val, double* rc,
+                        cudaStream_t s, hb::Prolong<double> pro = {})
+{
+    const LevelOpt* o = opt(A);
+    return hb::launch_small_zero<double>(o->st, o->diag, A.inv_diag, nullptr, const_cast<double*>(r), x, ell_val,
+                                         rc ? mgopt(A)->inj_c : nullptr, rc, s, pro);
+}
+
+int small_zero_restrict(const SparseMatrix& A, const double* r64, float* r, float* x, cudaStream_t s,
+                        hb::Prolong<float> pro = {})
+{
+    const LevelOpt* o = opt(A);
+    const MGOpt* mo = mgopt(A);
+    return hb::launch_small_zero<float>(o->st, o->diag32, o->inv_diag32, r64, r, x, nullptr, mo ? mo->inj_c : nullptr,
+                                        mo ? mo->rc32 : nullptr, s, pro);
+}
+
+// One full / zero-guess SymGS step on the ELL matrix.
+int symgs_ell(const SparseMatrix& A, const double* r, double* x, cudaStream_t s, hb::Prolong<double> pro = {})
+{
+    if(small_level<double>(A, true))
+        return hb::launch_small_symgs<double>(opt(A)->st, A.inv_diag, r, x, nullptr, A.ell_val, s, pro);
+    return hb::launch_symgs(A.localNumberOfRows, A.nblocks, A.ublocks, A.sizes, A.offsets, A.ell_col_ind, A.ell_val,
+                            A.inv_diag, r, x, s, pro);
+}
+
+int symgs_zero_ell(const SparseMatrix& A, const double* r, double* x, cudaStream_t s, hb::Prolong<double> pro = {})
+{
+    const LevelOpt* o = opt(A);
+    if(small_level<double>(A, true)) return small_zero_restrict(A, r, x, A.ell_val, nullptr, s, pro);
+    return hb::launch_symgs_zero(A.localNumberOfRows, A.nblocks, A.ublocks, A.sizes, A.offsets, A.ell_col_ind,
+                                 A.ell_val, A.diag_idx, o->diag, A.inv_diag, r, x, s, pro, zg_of(A));
+}
+
+}  // namespace
+
 // src/ComputeSYMGS.cpp:369-404.
 int ComputeSYMGS(const SparseMatrix& A, const Vector& r, Vector& x)
 {
     return guarded([&] {
         ExchangeHalo(A, x);
-        return hb::launch_symgs(A.localNumberOfRows, A.nblocks, A.ublocks, A.sizes, A.offsets, A.ell_col_ind,
-                                A.ell_val, A.inv_diag, r.d_values, x.d_values, rt().stream);
+        return symgs_ell(A, r.d_values, x.d_values, rt().stream);
     });
 }
 
 // src/ComputeSYMGS.cpp:406-454.
 int ComputeSYMGSZeroGuess(const SparseMatrix& A, const Vector& r, Vector& x)
 {
-    return guarded([&] {
-        return hb::launch_symgs_zero(A.localNumberOfRows, A.nblocks, A.ublocks, A.sizes, A.offsets, A.ell_col_ind,
-                                     A.ell_val, A.diag_idx, opt(A)->diag, A.inv_diag, r.d_values, x.d_values,
-                                     rt().stream, {}, zg_of(A));
-    });
+    return guarded([&] { return symgs_zero_ell(A, r.d_values, x.d_values, rt().stream); });
 }
 
 // src/ComputeRestriction.cpp:199-237.
@@ -110,21 +154,21 @@ namespace {
 int mg64_ell(const SparseMatrix& A, const Vector& r, Vector& x, hb::Prolong<double> pro)
 {
     cudaStream_t s = rt().stream;
-    const int m = A.localNumberOfRows;
-    auto zero_guess = [&](hb::Prolong<double> p) {
-        return hb::launch_symgs_zero(m, A.nblocks, A.ublocks, A.sizes, A.offsets, A.ell_col_ind, A.ell_val,
-                                     A.diag_idx, opt(A)->diag, A.inv_diag, r.d_values, x.d_values, s, p, zg_of(A));
-    };
+    auto zero_guess = [&](hb::Prolong<double> p) { return symgs_zero_ell(A, r.d_values, x.d_values, s, p); };
     auto full = [&](hb::Prolong<double> p) {
         ExchangeHalo(A, x);
-        return hb::launch_symgs(m, A.nblocks, A.ublocks, A.sizes, A.offsets, A.ell_col_ind, A.ell_val, A.inv_diag,
-                                r.d_values, x.d_values, s, p);
+        return symgs_ell(A, r.d_values, x.d_values, s, p);
     };
     if(!A.mgData) return zero_guess(pro);
     const int pre = A.mgData->numberOfPresmootherSteps, post = A.mgData->numberOfPostsmootherSteps;
-    HB_RETURN_IF(zero_guess(post == 0 ? pro : hb::Prolong<double>{}));
-    for(int i = 1; i < pre; ++i) HB_RETURN_IF(full({}));
-    HB_RETURN_IF(ComputeFusedSpMVRestriction(A, r, x));
+    if(pre == 1 && post > 0 && small_level<double>(A, true))
+        HB_RETURN_IF(small_zero_restrict(A, r.d_values, x.d_values, A.ell_val, A.mgData->rc->d_values, s));
+    else
+    {
+        HB_RETURN_IF(zero_guess(post == 0 ? pro : hb::Prolong<double>{}));
+        for(int i = 1; i < pre; ++i) HB_RETURN_IF(full({}));
+        HB_RETURN_IF(ComputeFusedSpMVRestriction(A, r, x));
+    }
     // src/ComputeMG.cpp:86-90: coarse solve, then ComputeProlongation -- here
     // carried out by the coarse level's final passes
     if(fused_prolongation())
@@ -155,10 +199,14 @@ int mg_fp32(const SparseMatrix& A, const float* r, float* x, cudaStream_t s, hb:
     const LevelOpt* o = opt(A);
     if(!A.mgData)
         return hb::launch32_symgs_zero(o->st, o->diag32, o->inv_diag32, nullptr, const_cast<float*>(r), x, s, pro);
-    HB_RETURN_IF(hb::launch32_symgs_zero(o->st, o->diag32, o->inv_diag32, nullptr, const_cast<float*>(r), x, s));
     const MGOpt* mo = mgopt(A);
     const int nc = A.Ac->localNumberOfRows;
-    HB_RETURN_IF(hb::launch32_restrict(o->st, nc, mo->inj_f, mo->inj_c, o->diag32, r, x, mo->rc32, s));
+    if(small_level<float>(A, false)) HB_RETURN_IF(small_zero_restrict(A, nullptr, const_cast<float*>(r), x, s));
+    else
+    {
+        HB_RETURN_IF(hb::launch32_symgs_zero(o->st, o->diag32, o->inv_diag32, nullptr, const_cast<float*>(r), x, s));
+        HB_RETURN_IF(hb::launch32_restrict(o->st, nc, mo->inj_f, mo->inj_c, o->diag32, r, x, mo->rc32, s));
+    }
     if(fused_prolongation()) HB_RETURN_IF(mg_fp32(*A.Ac, mo->rc32, mo->xc32, s, hb::Prolong<float>{x, mo->pro_f}));
     else
     {
@@ -184,11 +232,14 @@ int mg_mixed_to(const SparseMatrix& A, const double* r64, double* z64, cudaStrea
             return hb::record_error(HPCGB200_ERR_NOT_STENCIL,
                                     "mixed V-cycle needs the 27-point stencil in parity colouring on every level");
     const int m = A.localNumberOfRows;
-    HB_RETURN_IF(hb::launch32_symgs_zero(o->st, o->diag32, o->inv_diag32, r64, o->r32, o->z32, s));
+    const bool small = small_level<float>(A, false);
+    if(small) HB_RETURN_IF(small_zero_restrict(A, r64, o->r32, o->z32, s));
+    else HB_RETURN_IF(hb::launch32_symgs_zero(o->st, o->diag32, o->inv_diag32, r64, o->r32, o->z32, s));
     if(!A.mgData) return z64 ? hb::launch_cast_f2d(m, o->z32, z64, s) : 0;
     const MGOpt* mo = mgopt(A);
     const int nc = A.Ac->localNumberOfRows;
-    HB_RETURN_IF(hb::launch32_restrict(o->st, nc, mo->inj_f, mo->inj_c, o->diag32, o->r32, o->z32, mo->rc32, s));
+    if(!small)
+        HB_RETURN_IF(hb::launch32_restrict(o->st, nc, mo->inj_f, mo->inj_c, o->diag32, o->r32, o->z32, mo->rc32, s));
     if(fused_prolongation()) HB_RETURN_IF(mg_fp32(*A.Ac, mo->rc32, mo->xc32, s, hb::Prolong<float>{o->z32, mo->pro_f}));
     else
     {
@@ -219,21 +270,20 @@ bool stencil_vec_level(const SparseMatrix& A)
 int mg64_stencil(const SparseMatrix& A, const double* r, double* x, cudaStream_t s, hb::Prolong<double> pro)
 {
     const LevelOpt* o = opt(A);
-    const bool vec = stencil_vec_level(A);
+    const bool vec = stencil_vec_level(A), small = small_level<double>(A, false);
     // the coarsest level's zero-guess step is its last: it carries `pro`
     const hb::Prolong<double> pz = A.mgData ? hb::Prolong<double>{} : pro;
-    if(vec) HB_RETURN_IF(hb::launch64v_symgs_zero(o->st, o->diag, A.inv_diag, r, x, s, pz));
-    else
-        HB_RETURN_IF(hb::launch_symgs_zero(A.localNumberOfRows, A.nblocks, A.ublocks, A.sizes, A.offsets,
-                                           A.ell_col_ind, A.ell_val, A.diag_idx, o->diag, A.inv_diag, r, x, s, pz,
-                                           zg_of(A)));
+    if(small)
+        HB_RETURN_IF(small_zero_restrict(A, r, x, nullptr, A.mgData ? A.mgData->rc->d_values : nullptr, s, pz));
+    else if(vec) HB_RETURN_IF(hb::launch64v_symgs_zero(o->st, o->diag, A.inv_diag, r, x, s, pz));
+    else HB_RETURN_IF(symgs_zero_ell(A, r, x, s, pz));
     if(!A.mgData) return 0;
     const MGOpt* mo = mgopt(A);
     const int nc = A.Ac->localNumberOfRows;
     double* rc = A.mgData->rc->d_values;
     double* xc = A.mgData->xc->d_values;
-    if(vec) HB_RETURN_IF(hb::launch64v_restrict(o->st, nc, mo->inj_c, o->diag, r, x, rc, s));
-    else
+    if(!small && vec) HB_RETURN_IF(hb::launch64v_restrict(o->st, nc, mo->inj_c, o->diag, r, x, rc, s));
+    else if(!small)
         HB_RETURN_IF(hb::launch_restrict(nc, mo->inj_f, mo->inj_c, A.localNumberOfRows, A.ell_col_ind, A.ell_val, r, x,
                                          rc, s));
     // coarse solve with the prolongation into x fused into its final passes
@@ -244,9 +294,9 @@ int mg64_stencil(const SparseMatrix& A, const double* r, double* x, cudaStream_t
         if(vec) HB_RETURN_IF(hb::launch64v_prolong(o->st, nc, mo->inj_c, xc, x, s));
         else HB_RETURN_IF(hb::launch_prolong(nc, mo->inj_f, mo->inj_c, xc, x, s));
     }
+    if(small) return hb::launch_small_symgs<double>(o->st, A.inv_diag, r, x, nullptr, nullptr, s, pro);
     if(vec) return hb::launch64v_symgs(o->st, A.inv_diag, r, x, s, pro);
-    return hb::launch_symgs(A.localNumberOfRows, A.nblocks, A.ublocks, A.sizes, A.offsets, A.ell_col_ind, A.ell_val,
-                            A.inv_diag, r, x, s, pro);
+    return symgs_ell(A, r, x, s, pro);
 }
 
 }  // namespace
