@@ -312,98 +312,105 @@ inline dim3 brick_grid(const ColorLaunch& c)
     return dim3((unsigned)((c.bx + 31) / 32), (unsigned)((c.by + 7) / 8), (unsigned)c.bz);
 }
 
-template <bool kEven, bool kFromDouble>
-__global__ void __launch_bounds__(kBrickThreads) k32_fwd0(const ColorLaunch c, const StencilLevel L,
-                                                          const float* __restrict__ inv_diag32,
-                                                          const double* __restrict__ r64, float* __restrict__ r32,
-                                                          float* x, Prolong<float> pro)
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return fma(a, b, c); }
+
+// One row per thread, for levels whose colour bricks are not 4-aligned
+// (200 x 168 x 136: level 1 is 100 x 84 x 68, bricks of 50).  T = double is the
+// FP64 stencil V-cycle there: the ELL kernels it replaces read 12 B a slot.
+template <typename T, bool kEven, bool kFromDouble>
+__global__ void __launch_bounds__(kBrickThreads) k1_fwd0(const ColorLaunch c, const StencilLevel L,
+                                                         const T* __restrict__ inv_diag,
+                                                         const double* __restrict__ r64, T* __restrict__ r, T* x,
+                                                         Prolong<T> pro)
 {
     const BrickRow b = brick_row(c, blockIdx.z);
     if(!b.in) return;
     const int row = b.row;
-    float sum;
-    if(kFromDouble)
+    T sum;
+    if constexpr(kFromDouble)
     {
-        sum = (float)r64[row];
-        r32[row] = sum;
+        sum = (T)r64[row];
+        r[row] = sum;
     }
     else
     {
-        sum = r32[row];
+        sum = r[row];
     }
     if(c.tb.dp > 0)
     {
-        float val[27];
-        gather<kBefore, kEven>(L, c, b, x, -0.0f, val);
+        T val[27];
+        gather<kBefore, kEven>(L, c, b, x, T(-0.0), val);
 #pragma unroll
         for(int j = 0; j < 27; ++j) sum = sum + val[j];
     }
-    const float xn = sum * inv_diag32[row];
+    const T xn = sum * inv_diag[row];
     x[row] = xn;
     pro.add(row, xn);
 }
 
-template <bool kEven>
-__global__ void __launch_bounds__(kBrickThreads) k32_bwd0(const ColorLaunch c, const StencilLevel L,
-                                                          const float* __restrict__ diag32,
-                                                          const float* __restrict__ inv_diag32, float* x,
-                                                          Prolong<float> pro)
+template <typename T, bool kEven>
+__global__ void __launch_bounds__(kBrickThreads) k1_bwd0(const ColorLaunch c, const StencilLevel L,
+                                                         const T* __restrict__ diag, const T* __restrict__ inv_diag,
+                                                         T* x, Prolong<T> pro)
 {
     const BrickRow b = brick_row(c, blockIdx.z);
     if(!b.in) return;
     const int row = b.row;
-    float val[27];
-    gather<kAfter, kEven>(L, c, b, x, -0.0f, val);
-    float sum = __fmul_rn(x[row], diag32[row]);
+    T val[27];
+    gather<kAfter, kEven>(L, c, b, x, T(-0.0), val);
+    T sum = mul_rn(x[row], diag[row]);
 #pragma unroll
     for(int j = 0; j < 27; ++j) sum = sum + val[j];
-    const float xn = sum * inv_diag32[row];
+    const T xn = sum * inv_diag[row];
     x[row] = xn;
     pro.add(row, xn);
 }
 
-template <bool kEven>
-__global__ void __launch_bounds__(kBrickThreads) k32_sweep(const ColorLaunch c, const StencilLevel L,
-                                                           const float* __restrict__ inv_diag32,
-                                                           const float* __restrict__ r, float* x,
-                                                           double* __restrict__ z64, Prolong<float> pro)
+template <typename T, bool kEven>
+__global__ void __launch_bounds__(kBrickThreads) k1_sweep(const ColorLaunch c, const StencilLevel L,
+                                                          const T* __restrict__ inv_diag, const T* __restrict__ r,
+                                                          T* x, double* __restrict__ z64, Prolong<T> pro)
 {
     const BrickRow b = brick_row(c, blockIdx.z);
     if(!b.in) return;
     const int row = b.row;
-    float val[27];
-    gather<kOff, kEven>(L, c, b, x, -0.0f, val);
-    float sum = r[row];
+    T val[27];
+    gather<kOff, kEven>(L, c, b, x, T(-0.0), val);
+    T sum = r[row];
 #pragma unroll
     for(int j = 0; j < 27; ++j) sum = sum + val[j];
-    const float xn = sum * inv_diag32[row];
+    const T xn = sum * inv_diag[row];
     x[row] = xn;
-    if(z64) z64[row] = (double)xn;
+    if constexpr(sizeof(T) == 4)
+        if(z64) z64[row] = (double)xn;
     pro.add(row, xn);
 }
 
 // Residual at the injected rows (all of parity class 0: launch c is that colour).
-template <bool kEven>
-__global__ void __launch_bounds__(kBS32) k32_restrict(const ColorLaunch c, const StencilLevel L, int nc,
-                                                      const int* __restrict__ inj_f, const int* __restrict__ inj_c,
-                                                      const float* __restrict__ diag32, const float* __restrict__ rf,
-                                                      const float* __restrict__ xf, float* __restrict__ rc)
+template <typename T, bool kEven>
+__global__ void __launch_bounds__(kBS32) k1_restrict(const ColorLaunch c, const StencilLevel L, int nc,
+                                                     const int* __restrict__ inj_f, const int* __restrict__ inj_c,
+                                                     const T* __restrict__ diag, const T* __restrict__ rf,
+                                                     const T* __restrict__ xf, T* __restrict__ rc)
 {
     const int ic = blockIdx.x * kBS32 + threadIdx.x;
     const bool in = ic < nc;
     const BrickRow b = row_of(c, in ? inj_f[ic] : 0, in);
     if(!in) return;
     const int row = b.row;
-    float val[27];
-    gather<kOff, kEven>(L, c, b, xf, -0.0f, val);
-    const float dterm = -diag32[row];
-    const float xr = xf[row];
-    float sum = rf[row];
-    // ELL order: the diagonal term at slot dp (val[dp] is the no-op -0.0f)
+    T val[27];
+    gather<kOff, kEven>(L, c, b, xf, T(-0.0), val);
+    const T dterm = -diag[row];
+    const T xr = xf[row];
+    T sum = rf[row];
+    // ELL order: the diagonal term at slot dp (val[dp] is the no-op -0.0)
 #pragma unroll
     for(int j = 0; j < 27; ++j)
     {
-        if(j == c.tb.dp) sum = fmaf(dterm, xr, sum);
+        if(j == c.tb.dp) sum = fma_rn(dterm, xr, sum);
         sum = sum + val[j];
     }
     rc[inj_c[ic]] = sum;
@@ -508,11 +515,6 @@ struct Quad<double>
         *reinterpret_cast<double2*>(p + 2) = make_double2(v[2], v[3]);
     }
 };
-
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return fma(a, b, c); }
 
 template <typename T>
 __device__ __forceinline__ void ld4(const T* x, int i, int m, T (&v)[4])
@@ -2180,13 +2182,13 @@ int launch32_symgs_zero(const StencilLevel& L, const float* diag32, const float*
         }
         else if(L.even)
         {
-            if(r64) k32_fwd0<true, true><<<g, t, 0, s>>>(c, L, inv_diag32, r64, r32, x, pv);
-            else k32_fwd0<true, false><<<g, t, 0, s>>>(c, L, inv_diag32, nullptr, r32, x, pv);
+            if(r64) k1_fwd0<float, true, true><<<g, t, 0, s>>>(c, L, inv_diag32, r64, r32, x, pv);
+            else k1_fwd0<float, true, false><<<g, t, 0, s>>>(c, L, inv_diag32, nullptr, r32, x, pv);
         }
         else
         {
-            if(r64) k32_fwd0<false, true><<<g, t, 0, s>>>(c, L, inv_diag32, r64, r32, x, pv);
-            else k32_fwd0<false, false><<<g, t, 0, s>>>(c, L, inv_diag32, nullptr, r32, x, pv);
+            if(r64) k1_fwd0<float, false, true><<<g, t, 0, s>>>(c, L, inv_diag32, r64, r32, x, pv);
+            else k1_fwd0<float, false, false><<<g, t, 0, s>>>(c, L, inv_diag32, nullptr, r32, x, pv);
         }
         HB_LAUNCHED();
     }
@@ -2205,8 +2207,8 @@ int launch32_symgs_zero(const StencilLevel& L, const float* diag32, const float*
                 return launch_pdl(kv_bwd0<float, G, C>, brick_grid4(c), t4, s, c, L, diag32, inv_diag32, x, pro);
             }));
         }
-        else if(L.even) k32_bwd0<true><<<brick_grid(c), t, 0, s>>>(c, L, diag32, inv_diag32, x, pro);
-        else k32_bwd0<false><<<brick_grid(c), t, 0, s>>>(c, L, diag32, inv_diag32, x, pro);
+        else if(L.even) k1_bwd0<float, true><<<brick_grid(c), t, 0, s>>>(c, L, diag32, inv_diag32, x, pro);
+        else k1_bwd0<float, false><<<brick_grid(c), t, 0, s>>>(c, L, diag32, inv_diag32, x, pro);
         HB_LAUNCHED();
     }
     return 0;
@@ -2235,8 +2237,8 @@ int launch32_symgs(const StencilLevel& L, const float* inv_diag32, const float* 
                                   z, pv);
             }));
         }
-        else if(L.even) k32_sweep<true><<<brick_grid(c), dim3(32, 8), 0, s>>>(c, L, inv_diag32, r, x, z, pv);
-        else k32_sweep<false><<<brick_grid(c), dim3(32, 8), 0, s>>>(c, L, inv_diag32, r, x, z, pv);
+        else if(L.even) k1_sweep<float, true><<<brick_grid(c), dim3(32, 8), 0, s>>>(c, L, inv_diag32, r, x, z, pv);
+        else k1_sweep<float, false><<<brick_grid(c), dim3(32, 8), 0, s>>>(c, L, inv_diag32, r, x, z, pv);
         HB_LAUNCHED();
         return 0;
     };
@@ -2267,8 +2269,8 @@ int launch32_restrict(const StencilLevel& Lf, int nc, const int* inj_f, const in
                               xf, rc);
         }));
     }
-    else if(Lf.even) k32_restrict<true><<<nblk(nc), kBS32, 0, s>>>(c, Lf, nc, inj_f, inj_c, diag32, rf, xf, rc);
-    else k32_restrict<false><<<nblk(nc), kBS32, 0, s>>>(c, Lf, nc, inj_f, inj_c, diag32, rf, xf, rc);
+    else if(Lf.even) k1_restrict<float, true><<<nblk(nc), kBS32, 0, s>>>(c, Lf, nc, inj_f, inj_c, diag32, rf, xf, rc);
+    else k1_restrict<float, false><<<nblk(nc), kBS32, 0, s>>>(c, Lf, nc, inj_f, inj_c, diag32, rf, xf, rc);
     HB_LAUNCHED();
     return 0;
 }
@@ -2297,8 +2299,8 @@ bool stencil_vec4(const StencilLevel& L) { return vec4_ok(L); }
 int launch64v_symgs_zero(const StencilLevel& L, const double* diag, const double* inv_diag, const double* r,
                          double* x, cudaStream_t s, Prolong<double> pro)
 {
-    if(!vec4_ok(L)) return record_error(HPCGB200_ERR_ARG, "FP64 stencil V-cycle: colour bricks not 4-aligned");
-    const dim3 t4(kV4X, kV4Y);
+    const dim3 t4(kV4X, kV4Y), t1(32, 8);
+    const bool vec = vec4_ok(L);
     const std::shared_ptr<const SweepMaps> maps = pass_tma_ok(L, x, pro) ? sweep_maps(L, x) : nullptr;
     if(pass_tma_ok(L, x, pro) && !maps) return HPCGB200_ERR_CUDA;
     for(int v = 0; v < L.ncolors; ++v)
@@ -2310,6 +2312,14 @@ int launch64v_symgs_zero(const StencilLevel& L, const double* diag, const double
         {
             HB_CUDA((pass_tma<double, kTmaFwd0>(L, c, *maps, inv_diag, nullptr, nullptr, const_cast<double*>(r), x,
                                                 nullptr, s)));
+            continue;
+        }
+        if(!vec)
+        {
+            double* rr = const_cast<double*>(r);
+            if(L.even) k1_fwd0<double, true, false><<<brick_grid(c), t1, 0, s>>>(c, L, inv_diag, nullptr, rr, x, pv);
+            else k1_fwd0<double, false, false><<<brick_grid(c), t1, 0, s>>>(c, L, inv_diag, nullptr, rr, x, pv);
+            HB_LAUNCHED();
             continue;
         }
         HB_CUDA(by_shape<double>(L, c, [&](auto kg, auto kc) {
@@ -2327,6 +2337,13 @@ int launch64v_symgs_zero(const StencilLevel& L, const double* diag, const double
             HB_CUDA((pass_tma<double, kTmaBwd0>(L, c, *maps, inv_diag, diag, nullptr, nullptr, x, nullptr, s)));
             continue;
         }
+        if(!vec)
+        {
+            if(L.even) k1_bwd0<double, true><<<brick_grid(c), t1, 0, s>>>(c, L, diag, inv_diag, x, pro);
+            else k1_bwd0<double, false><<<brick_grid(c), t1, 0, s>>>(c, L, diag, inv_diag, x, pro);
+            HB_LAUNCHED();
+            continue;
+        }
         HB_CUDA(by_shape<double>(L, c, [&](auto kg, auto kc) {
             constexpr int G = decltype(kg)::value, C = decltype(kc)::value;
             return launch_pdl(kv_bwd0<double, G, C>, brick_grid4(c), t4, s, c, L, diag, inv_diag, x, pro);
@@ -2338,7 +2355,7 @@ int launch64v_symgs_zero(const StencilLevel& L, const double* diag, const double
 int launch64v_symgs(const StencilLevel& L, const double* inv_diag, const double* r, double* x, cudaStream_t s,
                     Prolong<double> pro)
 {
-    if(!vec4_ok(L)) return record_error(HPCGB200_ERR_ARG, "FP64 stencil V-cycle: colour bricks not 4-aligned");
+    const bool vec = vec4_ok(L);
     const std::shared_ptr<const SweepMaps> maps = pass_tma_ok(L, x, pro) ? sweep_maps(L, x) : nullptr;
     if(pass_tma_ok(L, x, pro) && !maps) return HPCGB200_ERR_CUDA;
     auto sweep = [&](int v, Prolong<double> pv) -> int {
@@ -2348,6 +2365,14 @@ int launch64v_symgs(const StencilLevel& L, const double* inv_diag, const double*
         {
             HB_CUDA((pass_tma<double, kTmaSweep>(L, c, *maps, inv_diag, nullptr, nullptr, const_cast<double*>(r), x,
                                                  nullptr, s)));
+            return 0;
+        }
+        if(!vec)
+        {
+            const dim3 t1(32, 8);
+            if(L.even) k1_sweep<double, true><<<brick_grid(c), t1, 0, s>>>(c, L, inv_diag, r, x, nullptr, pv);
+            else k1_sweep<double, false><<<brick_grid(c), t1, 0, s>>>(c, L, inv_diag, r, x, nullptr, pv);
+            HB_LAUNCHED();
             return 0;
         }
         HB_CUDA(by_shape<double>(L, c, [&](auto kg, auto kc) {
@@ -2362,12 +2387,17 @@ int launch64v_symgs(const StencilLevel& L, const double* inv_diag, const double*
     return 0;
 }
 
-int launch64v_restrict(const StencilLevel& Lf, int nc, const int* inj_c, const double* diag, const double* rf,
-                       const double* xf, double* rc, cudaStream_t s)
+int launch64v_restrict(const StencilLevel& Lf, int nc, const int* inj_f, const int* inj_c, const double* diag,
+                       const double* rf, const double* xf, double* rc, cudaStream_t s)
 {
     const ColorLaunch c = color_launch(Lf, Lf.color_of_par[0]);
     if(!vec4_ok(Lf) || nc != c.bx * c.by * c.bz)
-        return record_error(HPCGB200_ERR_ARG, "FP64 stencil restriction: colour bricks not 4-aligned");
+    {
+        if(Lf.even) k1_restrict<double, true><<<nblk(nc), kBS32, 0, s>>>(c, Lf, nc, inj_f, inj_c, diag, rf, xf, rc);
+        else k1_restrict<double, false><<<nblk(nc), kBS32, 0, s>>>(c, Lf, nc, inj_f, inj_c, diag, rf, xf, rc);
+        HB_LAUNCHED();
+        return 0;
+    }
     if(pass_tma_ok(Lf, xf, Prolong<double>{}))
     {
         const std::shared_ptr<const SweepMaps> maps = sweep_maps(Lf, xf);

@@ -266,23 +266,25 @@ bool stencil_vec_level(const SparseMatrix& A)
 
 // ComputeMG's recursion (1 zero-guess pre-smoothing step, fused restriction,
 // coarse solve, prolongation, 1 post-smoothing step) per level on the
-// implicit-stencil kernels or, where the bricks are not 4-aligned, the ELL ones.
+// implicit-stencil kernels or, where the level is not the verified stencil,
+// the ELL ones.
 int mg64_stencil(const SparseMatrix& A, const double* r, double* x, cudaStream_t s, hb::Prolong<double> pro)
 {
     const LevelOpt* o = opt(A);
-    const bool vec = stencil_vec_level(A), small = small_level<double>(A, false);
+    const bool stencil = o && o->stencil_ok, vec = stencil_vec_level(A), small = small_level<double>(A, false);
     // the coarsest level's zero-guess step is its last: it carries `pro`
     const hb::Prolong<double> pz = A.mgData ? hb::Prolong<double>{} : pro;
     if(small)
         HB_RETURN_IF(small_zero_restrict(A, r, x, nullptr, A.mgData ? A.mgData->rc->d_values : nullptr, s, pz));
-    else if(vec) HB_RETURN_IF(hb::launch64v_symgs_zero(o->st, o->diag, A.inv_diag, r, x, s, pz));
+    else if(stencil) HB_RETURN_IF(hb::launch64v_symgs_zero(o->st, o->diag, A.inv_diag, r, x, s, pz));
     else HB_RETURN_IF(symgs_zero_ell(A, r, x, s, pz));
     if(!A.mgData) return 0;
     const MGOpt* mo = mgopt(A);
     const int nc = A.Ac->localNumberOfRows;
     double* rc = A.mgData->rc->d_values;
     double* xc = A.mgData->xc->d_values;
-    if(!small && vec) HB_RETURN_IF(hb::launch64v_restrict(o->st, nc, mo->inj_c, o->diag, r, x, rc, s));
+    if(!small && stencil)
+        HB_RETURN_IF(hb::launch64v_restrict(o->st, nc, mo->inj_f, mo->inj_c, o->diag, r, x, rc, s));
     else if(!small)
         HB_RETURN_IF(hb::launch_restrict(nc, mo->inj_f, mo->inj_c, A.localNumberOfRows, A.ell_col_ind, A.ell_val, r, x,
                                          rc, s));
@@ -295,7 +297,7 @@ int mg64_stencil(const SparseMatrix& A, const double* r, double* x, cudaStream_t
         else HB_RETURN_IF(hb::launch_prolong(nc, mo->inj_f, mo->inj_c, xc, x, s));
     }
     if(small) return hb::launch_small_symgs<double>(o->st, A.inv_diag, r, x, nullptr, nullptr, s, pro);
-    if(vec) return hb::launch64v_symgs(o->st, A.inv_diag, r, x, s, pro);
+    if(stencil) return hb::launch64v_symgs(o->st, A.inv_diag, r, x, s, pro);
     return symgs_ell(A, r, x, s, pro);
 }
 
