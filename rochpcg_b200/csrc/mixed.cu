@@ -2527,8 +2527,10 @@ int launch_cg_step1_sep(const StencilLevel& L, const double* diag, const double*
     static const int grid_tma = resident_grid(k_cg_step1_sep<float, true>, kMThreads, kReduceBlocks);
     static const int grid_cp = resident_grid(k_cg_step1_sep<float, false>, kMThreads, kReduceBlocks);
     const std::shared_ptr<const SepMaps> M = sep_tma_maps(L, p);
-    const int grid = M ? grid_tma : grid_cp;
-    if(grid <= 0) return record_error(HPCGB200_ERR_CUDA, "CG step: no resident grid");
+    const int resident = M ? grid_tma : grid_cp;
+    if(resident <= 0) return record_error(HPCGB200_ERR_CUDA, "CG step: no resident grid");
+    const dim3 tiles = sep_grid(L);
+    const int grid = step1_grid(resident, L.m, (long long)tiles.x * tiles.y * tiles.z, kMThreads);
     if(M)
         HB_CUDA(launch_coop(k_cg_step1_sep<float, true>, grid, kMThreads, s, L, diag, r, z, p, x, Ap, st, ws->partial,
                             &ws->ticket, gb, *M));
