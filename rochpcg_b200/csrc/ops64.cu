@@ -331,11 +331,10 @@ __global__ void k_diag_bounds(int lo, int hi, const int* __restrict__ diag_idx, 
     }
 }
 
-int zero_guess_groups(int m, int nblocks, const int* offsets, const int* diag_idx, ZgGroups* zg, cudaStream_t s)
+int zero_guess_groups(int m, int nblocks, const int* offsets, const int* diag_idx, ZgGroups* zg, int* d,
+                      cudaStream_t s)
 {
     if(nblocks <= 0) return 0;
-    int* d = nullptr;
-    HB_CUDA(cudaMallocAsync(&d, sizeof(int) * 2 * nblocks, s));
     std::vector<int> init(2 * nblocks), h(2 * nblocks);
     for(int c = 0; c < nblocks; ++c) init[2 * c] = kWidth, init[2 * c + 1] = 0;
     HB_CUDA(cudaMemcpyAsync(d, init.data(), sizeof(int) * 2 * nblocks, cudaMemcpyHostToDevice, s));
@@ -349,7 +348,6 @@ int zero_guess_groups(int m, int nblocks, const int* offsets, const int* diag_id
     }
     HB_CUDA(cudaMemcpyAsync(h.data(), d, sizeof(int) * 2 * nblocks, cudaMemcpyDeviceToHost, s));
     HB_CUDA(cudaStreamSynchronize(s));
-    HB_CUDA(cudaFreeAsync(d, s));
     (void)m;
     for(int c = 0; c < nblocks; ++c)
     {

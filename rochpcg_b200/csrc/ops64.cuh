@@ -109,8 +109,9 @@ int launch_symgs_zero(int m, int nblocks, int ublocks, const int* sizes, const i
                       const double* r, double* x, cudaStream_t s, Prolong<double> pro = {},
                       const ZgGroups* zg = nullptr);
 // The group ranges of colours [0, nblocks) from their rows' diagonal slots
-// (synchronizes the stream).
-int zero_guess_groups(int m, int nblocks, const int* offsets, const int* diag_idx, ZgGroups* zg, cudaStream_t s);
+// (scratch: 2 * nblocks device ints; synchronizes the stream).
+int zero_guess_groups(int m, int nblocks, const int* offsets, const int* diag_idx, ZgGroups* zg, int* scratch,
+                      cudaStream_t s);
 // pro_f[inj_c[ic]] = inj_f[ic]: coarse permuted row -> injected fine permuted row.
 int launch_prolong_map(int nc, const int* inj_f, const int* inj_c, int* pro_f, cudaStream_t s);
 int launch_restrict(int nc, const int* inj_f, const int* inj_c, int mf, const int* ell_col, const double* ell_val,

@@ -22,7 +22,7 @@ using namespace hpcg_b200;
 
 namespace hpcg_b200 {
 
-static void ensure_state(LevelOpt* o, int max_iter)
+void ensure_state(LevelOpt* o, int max_iter)
 {
     if(!o->step_barrier) o->step_barrier = dalloc<hb::GridBarrier>(1);
     if(o->cg_state && o->cg_state_iters >= max_iter) return;

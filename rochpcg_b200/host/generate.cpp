@@ -120,11 +120,11 @@ void GenerateProblem(SparseMatrix& A, Vector* b, Vector* x, Vector* xexact)
     if(x) CudaInitializeVector(*x, m);
     if(xexact) CudaInitializeVector(*xexact, m);
 
-    A.d_mtxIndL = dalloc<local_int_t>(slots);
-    A.d_matrixValues = dalloc<double>(slots);
+    A.d_mtxIndL = dalloc<local_int_t>(slots, kTemporary);
+    A.d_matrixValues = dalloc<double>(slots, kTemporary);
     A.d_nonzerosInRow = dalloc<char>(m);
     A.d_matrixDiagonal = dalloc<local_int_t>(m);
-    A.d_rowHash = dalloc<local_int_t>(m);
+    A.d_rowHash = dalloc<local_int_t>(m, kTemporary);
     A.d_localToGlobalMap = dalloc<global_int_t>(m);
 
     check(hpcgb200_generate_problem(nx, ny, nz, A.geom->gnx, A.geom->gny, A.geom->gnz, A.geom->gix0, A.geom->giy0,

@@ -97,13 +97,45 @@ int guarded(F&& f)
     }
 }
 
-template <typename T>
-T* dalloc(size_t n)
+// ---- device memory of a problem under construction
+// cudaMalloc and cudaFree cost 0.2-1 ms each, and a problem has about 100
+// arrays: 128^3 took 27 ms to create, of which 2.5 ms were kernels, and 13 ms to
+// destroy; with chunks 12 and 3 ms.  While an
+// ArenaScope is alive on a thread, that thread's allocations below
+// kArenaLargest come from chunks: one kind for what stays with the problem, one
+// for what set-up frees again.  A chunk goes back to the driver when its last
+// array is freed (dfree, any thread) and no scope fills it any more, so nothing
+// outlives the problem; the unused rest of a chunk is the only extra memory.
+enum AllocKind
 {
-    void* p = nullptr;
-    if(n == 0) n = 1;
-    HB_HOST_CUDA(cudaMalloc(&p, n * sizeof(T)));
-    return static_cast<T*>(p);
+    kKept = 0,
+    kTemporary = 1
+};
+constexpr size_t kArenaLargest = 32u << 20, kArenaChunk = 256u << 20;
+
+class ArenaScope
+{
+public:
+    // rows: level-0 rows of the problem (sizes the first chunk)
+    explicit ArenaScope(long long rows);
+    ~ArenaScope();
+    ArenaScope(const ArenaScope&) = delete;
+    ArenaScope& operator=(const ArenaScope&) = delete;
+    void* take(size_t bytes, AllocKind kind);  // nullptr: does not fit, or no memory for a chunk
+
+private:
+    char* chunk_[2] = {nullptr, nullptr};      // being filled
+    size_t next_[2];                           // capacity of the next one
+    ArenaScope* outer_;
+};
+
+// cudaMalloc, or a piece of the thread's arena; throws Error.
+void* device_alloc(size_t bytes, AllocKind kind);
+
+template <typename T>
+T* dalloc(size_t n, AllocKind kind = kKept)
+{
+    return static_cast<T*>(device_alloc((n ? n : 1) * sizeof(T), kind));
 }
 void dfree(void* p);
 
@@ -205,6 +237,9 @@ int mg_fp32(const SparseMatrix& A, const float* r, float* x, cudaStream_t s, hb:
 // result is left in opt(A)->z32, and also written to z64 when it is not null.
 int mg_mixed_to(const SparseMatrix& A, const double* r64, double* z64, cudaStream_t s);
 int mg_learned_to(const SparseMatrix& A, const double* r64, double* z64, cudaStream_t s);
+
+// The solver state of level 0 (o) with room for max_iter iterations, defined in cg.cpp.
+void ensure_state(LevelOpt* o, int max_iter);
 
 // Kernel launches of one CG iteration (captures the iteration graph if it
 // does not exist yet; nothing is launched), defined in cg.cpp.

@@ -33,7 +33,7 @@ static void optimize_level(SparseMatrix& A)
     A.perm = dalloc<local_int_t>(m);
     o->colors = dalloc<int>(m);
     const size_t wsb = hpcgb200_coloring_workspace_bytes(m);
-    void* ws = dalloc<char>(wsb);
+    void* ws = dalloc<char>(wsb, kTemporary);
     A.sizes = new local_int_t[HPCGB200_MAX_COLORS];
     A.offsets = new local_int_t[HPCGB200_MAX_COLORS + 1];
     int jpl_blocks = 0;
@@ -59,7 +59,10 @@ static void optimize_level(SparseMatrix& A)
     A.inv_diag = dalloc<double>(m);
     o->diag = dalloc<double>(m);
     check(hpcgb200_extract_diagonal(m, A.ell_col_ind, A.ell_val, A.diag_idx, A.inv_diag, o->diag, s));
-    check(hb::zero_guess_groups(m, A.nblocks, A.offsets, A.diag_idx, o->zg, s));
+    int* bounds = dalloc<int>(2 * HPCGB200_MAX_COLORS, kTemporary);
+    rc = hb::zero_guess_groups(m, A.nblocks, A.offsets, A.diag_idx, o->zg, bounds, s);
+    dfree(bounds);
+    check(rc);
     o->zg_ok = true;
     o->cc = hb::make_chunks(m, A.nblocks, A.offsets);
 
@@ -80,7 +83,7 @@ static void optimize_level(SparseMatrix& A)
         ok = hb::make_stencil_level(nx, ny, nz, A.offsets, cop, &o->st);
         if(ok)
         {
-            int* bad = dalloc<int>(1);
+            int* bad = dalloc<int>(1, kTemporary);
             HB_HOST_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), s));
             check(hb::launch_stencil_check(o->st, A.perm, A.ell_col_ind, A.ell_val, bad, s));
             int hbad = -1;
@@ -145,7 +148,7 @@ int OptimizeProblem(SparseMatrix& A, CGData& data, Vector& b, Vector& x, Vector&
 
         // permute b and xexact into the coloured order
         const local_int_t m = A.localNumberOfRows;
-        double* tmp = dalloc<double>(m);
+        double* tmp = dalloc<double>(m, kTemporary);
         check(hpcgb200_permute_vector(m, A.perm, b.d_values, tmp, s));
         HB_HOST_CUDA(cudaMemcpyAsync(b.d_values, tmp, sizeof(double) * m, cudaMemcpyDeviceToDevice, s));
         check(hpcgb200_permute_vector(m, A.perm, xexact.d_values, tmp, s));
@@ -168,6 +171,7 @@ int OptimizeProblem(SparseMatrix& A, CGData& data, Vector& b, Vector& x, Vector&
         HB_HOST_CUDA(cudaMemsetAsync(o->spmv_ticket, 0, sizeof(unsigned int), s));
 
         if(!data.r.d_values) CudaInitializeSparseCGData(A, data);
+        ensure_state(o, 1);
         for(SparseMatrix* M = &A; M; M = M->Ac) free_generated(*M);
         HB_HOST_CUDA(cudaStreamSynchronize(s));
         return 0;

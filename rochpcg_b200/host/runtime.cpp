@@ -2,8 +2,11 @@
 // Mirrors the reference's globals stream_interior / workspace
 // (src/utils.hpp:38-45, created in src/init.cpp:200-230) and the vector
 // helpers of src/Vector.hpp / src/CGData.hpp.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <mutex>
 
 #include "hpcg_b200.h"
 #include "internal.hpp"
@@ -26,9 +29,119 @@ void check_cuda(cudaError_t e, const char* what)
     }
 }
 
+namespace {
+
+struct Chunk
+{
+    size_t bytes, used;
+    int live;   // arrays not yet freed
+    bool open;  // a scope may still place arrays in it
+};
+
+std::mutex g_chunks_mutex;
+std::map<char*, Chunk> g_chunks;  // by base address
+thread_local ArenaScope* t_arena = nullptr;
+
+// Called with the mutex held: the chunk no scope fills any more.
+char* close_chunk(char* base)
+{
+    if(!base) return nullptr;
+    const auto it = g_chunks.find(base);
+    it->second.open = false;
+    if(it->second.live > 0) return nullptr;
+    g_chunks.erase(it);
+    return base;  // empty: the caller frees it
+}
+
+}  // namespace
+
+ArenaScope::ArenaScope(long long rows) : outer_(t_arena)
+{
+    // kept per level-0 row of a problem whose vectors go into chunks: about 140 B on level 0 and
+    // 50 for the coarse levels; of a larger one only the coarse levels' arrays do
+    const size_t kept = rows * 8 < (long long)kArenaLargest ? (size_t)rows * 190 : 64u << 20;
+    next_[kKept] = std::min(kArenaChunk, kept + (1u << 20));
+    next_[kTemporary] = std::min<size_t>(kArenaChunk / 4, (size_t)rows * 48 + (1u << 20));
+    t_arena = this;
+}
+
+ArenaScope::~ArenaScope()
+{
+    t_arena = outer_;
+    for(char* base : chunk_)
+    {
+        char* empty;
+        {
+            std::lock_guard<std::mutex> lock(g_chunks_mutex);
+            empty = close_chunk(base);
+        }
+        if(empty) cudaFree(empty);
+    }
+}
+
+void* ArenaScope::take(size_t bytes, AllocKind kind)
+{
+    bytes = (bytes + 255) & ~(size_t)255;
+    char* empty = nullptr;
+    char* p = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(g_chunks_mutex);
+        Chunk* c = chunk_[kind] ? &g_chunks[chunk_[kind]] : nullptr;
+        if(!c || c->used + bytes > c->bytes)
+        {
+            void* base = nullptr;
+            const size_t size = std::max(next_[kind], bytes);
+            if(cudaMalloc(&base, size) != cudaSuccess)
+            {
+                cudaGetLastError();
+                return nullptr;
+            }
+            empty = close_chunk(chunk_[kind]);
+            chunk_[kind] = static_cast<char*>(base);
+            c = &(g_chunks[chunk_[kind]] = Chunk{size, 0, 0, true});
+            next_[kind] = std::max<size_t>(2u << 20, next_[kind] / 4);
+        }
+        p = chunk_[kind] + c->used;
+        c->used += bytes;
+        ++c->live;
+    }
+    if(empty) cudaFree(empty);
+    return p;
+}
+
+void* device_alloc(size_t bytes, AllocKind kind)
+{
+    if(t_arena && bytes < kArenaLargest)
+        if(void* p = t_arena->take(bytes, kind)) return p;
+    void* p = nullptr;
+    HB_HOST_CUDA(cudaMalloc(&p, bytes));
+    return p;
+}
+
 void dfree(void* p)
 {
-    if(p) cudaFree(p);
+    if(!p) return;
+    {
+        std::lock_guard<std::mutex> lock(g_chunks_mutex);
+        auto it = g_chunks.upper_bound(static_cast<char*>(p));
+        if(it != g_chunks.begin())
+        {
+            --it;
+            Chunk& c = it->second;
+            if(static_cast<char*>(p) < it->first + c.bytes)
+            {
+                if(--c.live > 0) return;
+                if(c.open)
+                {
+                    c.used = 0;  // set-up work is stream ordered: the next arrays may take its place
+                    return;
+                }
+                p = it->first;
+                g_chunks.erase(it);
+            }
+        }
+    }
+    cudaFree(p);
 }
 
 void ensure_runtime()

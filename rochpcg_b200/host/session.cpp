@@ -113,6 +113,7 @@ extern "C" int hpcgb200_problem_create_ex(int nx, int ny, int nz, int nlevels, i
     auto* P = new hpcgb200_problem;
     const int rc = guarded([&] {
         g_keep_generated = (flags & HPCGB200_FLAG_KEEP_GENERATED) != 0;
+        ArenaScope arena((long long)nx * ny * nz);
         TracePhases trace;
         trace.phase("hpcg:GenerateProblem");
         const auto t0 = std::chrono::steady_clock::now();
