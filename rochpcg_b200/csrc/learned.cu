@@ -150,6 +150,26 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
     for(int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Four groups of four columns, `stride` columns apart.
+__device__ __forceinline__ void tmem_ld4x4(uint32_t taddr, uint32_t stride, float (&v)[4][4])
+{
+    uint32_t r[4][4];
+#pragma unroll
+    for(int k = 0; k < 4; ++k)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[k][0]), "=r"(r[k][1]), "=r"(r[k][2]), "=r"(r[k][3])
+                     : "r"(taddr + k * stride));
+    // the values as operands: nothing that uses them moves above the wait
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0][0]), "+r"(r[0][1]), "+r"(r[0][2]), "+r"(r[0][3]), "+r"(r[1][0]), "+r"(r[1][1]),
+                   "+r"(r[1][2]), "+r"(r[1][3]), "+r"(r[2][0]), "+r"(r[2][1]), "+r"(r[2][2]), "+r"(r[2][3]),
+                   "+r"(r[3][0]), "+r"(r[3][1]), "+r"(r[3][2]), "+r"(r[3][3])::"memory");
+#pragma unroll
+    for(int k = 0; k < 4; ++k)
+#pragma unroll
+        for(int i = 0; i < 4; ++i) v[k][i] = __uint_as_float(r[k][i]);
+}
+
 }  // namespace tc
 
 using namespace tc;
@@ -207,8 +227,10 @@ __host__ __device__ constexpr int weight_slot(int t) { return ((t / 3) % 3) * 9 
 //   warp 1      TMEM owner and MMA issuer: 3 (kTZ + 2) + kTZ - 1 MMAs per
 //               brick (21 for kTZ = 4) into one of two accumulators of
 //               kTZ x 48 columns;
-//   warps 2-5   epilogue: tcgen05.ld of the finished accumulator, the dx
-//               combination, ReLU / mask / permuted scatter, global stores.
+//   warps 2-9   epilogue: tcgen05.ld of the finished accumulator, the dx
+//               combination, ReLU / mask / permuted scatter, global stores
+//               (eight warps instead of four: a training batch, whose masked
+//               passes read the activations too, 371 -> 361 us).
 // Stage and accumulator hand-offs are mbarriers (TMA complete_tx, MMA commit,
 // epilogue arrivals), so loads, MMAs and stores of consecutive bricks overlap.
 
@@ -232,8 +254,10 @@ constexpr int kStages = HB_CONV_STAGES;
 constexpr int kPlaneCols = 3 * kNetCh;                // one output plane: 3 dx blocks of 16 channels
 constexpr int kAccCols = kTZ * kPlaneCols;            // FP32 columns of one brick's accumulator (192)
 constexpr int kTmemCols = 512;                        // two accumulators, rounded to a power of two
-constexpr int kConvThreads = 192;
-constexpr int kEpiThreads = 128;
+constexpr int kEpiWarps = 8;                          // two per TMEM lane quadrant, half of the planes each
+constexpr int kEpiThreads = 32 * kEpiWarps;
+constexpr int kConvThreads = 64 + kEpiThreads;
+static_assert(kTZ % 2 == 0, "planes per epilogue warp");
 constexpr int kConvSmem = kStages * kStageBytes + kNetWeightTileBytes + 256 + 1024;
 
 static_assert(kRowBytes == 32, "one point per 32-byte swizzle row (K = 16 per MMA)");
@@ -458,6 +482,8 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
         // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31
         const int qd = warp & 3;
         const int m = qd * 32 + lane;
+        constexpr int kPlanes = kTZ / 2;
+        const int mt0 = (warp - 2) / 4 * kPlanes;  // this warp's output planes of a brick
         long i = 0;
         for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++i)
         {
@@ -469,37 +495,34 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
             const int xi = m % kTX;
             const int x = bk.x0 - 1 + xi, y = bk.y0 + m / kTX;
             const bool halo = xi == 0 || xi == kTX - 1;
-            // masked output: the row's activations, one plane ahead, the first
-            // while the brick's MMAs run (loaded where they are used they cost
-            // a memory round trip a plane: 55 us against 27 unmasked on
-            // 2 x 64 samples of 16^3)
-            uint4 mask[2] = {};
-            auto load_mask = [&](int mt) {
-                const int z = bk.z0 + mt;
-                if(halo || x >= g.nx || y >= g.ny || z >= g.nz) return;
-                const uint4* ap = reinterpret_cast<const uint4*>(
-                    act + ((((long)bk.b * g.nz + z) * g.ny + y) * g.nx + x) * kNetCh);
-                mask[0] = __ldg(ap);
-                mask[1] = __ldg(ap + 1);
-            };
-            if constexpr(kOut == kOutMaskBf16) load_mask(0);
+            // masked output: the row's activations of the whole brick, loaded while
+            // its MMAs run (loaded where they are used they cost a memory round
+            // trip a plane: 55 us against 27 unmasked on 2 x 64 samples of 16^3)
+            uint4 mask[kOut == kOutMaskBf16 ? 2 * kPlanes : 1];
+            if constexpr(kOut == kOutMaskBf16)
+            {
+#pragma unroll
+                for(int mt = 0; mt < kPlanes; ++mt)
+                {
+                    const int z = bk.z0 + mt0 + mt;
+                    mask[2 * mt] = mask[2 * mt + 1] = make_uint4(0, 0, 0, 0);
+                    if(halo || x >= g.nx || y >= g.ny || z >= g.nz) continue;
+                    const uint4* ap = reinterpret_cast<const uint4*>(
+                        act + ((((long)bk.b * g.nz + z) * g.ny + y) * g.nx + x) * kNetCh);
+                    mask[2 * mt] = __ldg(ap);
+                    mask[2 * mt + 1] = __ldg(ap + 1);
+                }
+            }
             if(!role_wait(&tfull[acc], aph, abort_flag, status, 6)) break;
             tc_fence_after();
-#pragma unroll 1
-            for(int mt = 0; mt < kTZ; ++mt)
+#pragma unroll(kOut == kOutMaskBf16 ? kPlanes : 1)
+            for(int mt = 0; mt < kPlanes; ++mt)
             {
                 // out(x) = D_{dx=-1}[x - 1] + D_{dx=0}[x] + D_{dx=+1}[x + 1]: rows
                 // x +- 1 are the neighbouring lanes of the same 16-lane line
                 float dm[16], dc[16], dp[16], v[16];
-                __align__(16) __nv_bfloat16 h[16];
-                if constexpr(kOut == kOutMaskBf16)
-                {
-                    *reinterpret_cast<uint4*>(h) = mask[0];
-                    *reinterpret_cast<uint4*>(h + 8) = mask[1];
-                    if(mt + 1 < kTZ) load_mask(mt + 1);
-                }
                 const uint32_t ta =
-                    tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(acc * kAccCols + mt * kPlaneCols);
+                    tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(acc * kAccCols + (mt0 + mt) * kPlaneCols);
                 tmem_ld16(ta, dm);
                 tmem_ld16(ta + kNetCh, dc);
                 tmem_ld16(ta + 2 * kNetCh, dp);
@@ -510,7 +533,7 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
                     const float right = __shfl_down_sync(0xffffffffu, dp[c], 1);
                     v[c] = (left + dc[c]) + right;
                 }
-                const int z = bk.z0 + mt;
+                const int z = bk.z0 + mt0 + mt;
                 if(halo || x >= g.nx || y >= g.ny || z >= g.nz) continue;
                 const long p = (((long)bk.b * g.nz + z) * g.ny + y) * g.nx + x;
                 if constexpr(kOut == kOutReluBf16 || kOut == kOutMaskBf16)
@@ -522,6 +545,9 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
                     }
                     else
                     {
+                        __align__(16) __nv_bfloat16 h[16];
+                        *reinterpret_cast<uint4*>(h) = mask[2 * mt];
+                        *reinterpret_cast<uint4*>(h + 8) = mask[2 * mt + 1];
 #pragma unroll
                         for(int c = 0; c < 16; ++c) v[c] = __bfloat162float(h[c]) > 0.f ? v[c] : 0.f;
                     }
@@ -559,63 +585,39 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
 
 // ------------------------------------------------------------ layer 3 (16 -> 1)
 //
-// One output channel: the 27 taps are stacked in N instead of the input being
-// shifted.  For each staged input point p, ONE MMA row computes
-// D[p][t] = sum_c a2[p][c] w3[t][c] for all taps t (M = 128 points, N = 32,
-// K = 16), and the output is y[o] = sum_t D[o + off_t][t], gathered by the
-// epilogue from shared memory in tap order (deterministic, no atomics).  In
-// the odd evaluation the pair is folded into K: the branch of -r is a second
-// MMA into the same accumulator with the weights negated, both halved, so D
-// already holds (y(r) - y(-r)) / 2.
-//   warp 0      TMA producer: per brick one (two with the pair) box of the
-//               halo'd input, 18 x 10 x 4 points of 16 channels, 32-byte
-//               swizzled rows, zero fill outside the grid;
-//   warp 1      TMEM owner and MMA issuer: 6 MMAs (12 with the pair) per brick
-//               into one of two accumulators of 6 x 32 columns;
-//   warps 2-5   epilogue: TMEM -> shared memory (27 floats per staged point),
-//               then the 27-tap gather for the brick's 16 x 8 x 2 outputs.
-constexpr int k3X = 16, k3Y = 8, k3Z = 2;                       // output brick
-constexpr int k3HX = k3X + 2, k3HY = k3Y + 2, k3HZ = k3Z + 2;  // staged box 18 x 10 x 4
-constexpr int k3Rows = k3HX * k3HY * k3HZ;                      // 720 staged points
-constexpr int k3Chunks = (k3Rows + 127) / 128;                  // 6 M tiles per box
-constexpr int k3BoxBytes = k3Chunks * 128 * kRowBytes;          // 24 KB (the TMA fills the first 720 rows)
+// What bounds it: reading the two branches' activations (64 B a point of the
+// odd pair).  The 14 x 8 x 4 bricks, boxes, MMA plan and lane shuffles are the
+// 16 -> 16 convolution's with one output channel: a plane's accumulator is a
+// group of 16 columns of which dx = -1, 0, +1 take three, and every staged plane q
+// and row shift dy is ONE MMA for the 1-3 output planes it feeds (N = 16, 32 or
+// 48; 21 a brick, 42 with the pair).  In the odd evaluation the branch of -r
+// multiplies the negated weights, both halved, so the accumulator already holds
+// (y(r) - y(-r)) / 2.  The epilogue is one small tcgen05.ld and two lane shuffles
+// per output plane.  (All 27 taps in N with the sums gathered from shared
+// memory, 27 floats a staged point, was bound by that gather: 120 us on an odd
+// 128^3 sample; this form takes about 75, the boxes' 32-byte rows now the bound.
+// The whole network there: 301 -> 252 us; 256^3 learned V-cycle 661 -> 651 us.)
+//   warp 0      TMA producer: per brick one (two with the pair) box;
+//   warp 1      TMEM owner and MMA issuer, two accumulators of 4 x 16 columns;
+//   warps 2-5   epilogue.
+constexpr int k3EpiThreads = 128;
+constexpr int k3Threads = 64 + k3EpiThreads;
+constexpr int k3Stages = 3;
+constexpr int k3BoxBytes = kStageBytes;
 constexpr int k3StageBytes = 2 * k3BoxBytes;                    // the two branches of the pair
-constexpr int k3Stages = 2;
-constexpr int k3N = 32;                                         // 27 taps + 5 zero columns
-constexpr int k3AccCols = k3Chunks * k3N;                       // 192 TMEM columns per brick
-constexpr int k3TmemCols = 512;                                 // two accumulators, power of two
-constexpr int k3DStride = 27;                                   // floats per staged point (odd: no bank conflicts)
-constexpr int k3WTileBytes = k3N * kRowBytes;                   // 32 tap rows x 16 channels, K-major
-constexpr int k3Outputs = k3X * k3Y * k3Z;                      // 256 per brick
-constexpr int k3Smem = k3Stages * k3StageBytes + 2 * k3WTileBytes + k3Rows * k3DStride * 4 + 256 + 1024;
+constexpr int k3PlaneCols = 16;                                 // 3 dx and 13 zero columns (MMA N is a multiple of 16)
+constexpr int k3AccCols = kTZ * k3PlaneCols;
+constexpr int k3TmemCols = 2 * k3AccCols;
+constexpr int k3Tile = k3PlaneCols * kRowBytes;                 // 16 columns x 16 channels, K-major
+constexpr int k3Tiles = 9;                                      // [dy][dz = +1, 0, -1]
+constexpr int k3Smem = k3Stages * k3StageBytes + 2 * k3Tiles * k3Tile + 256 + 1024;
+static_assert(kTZ == 4, "tmem_ld4x4 reads the four planes");
 
-static_assert(k3BoxBytes % 1024 == 0 && k3Rows * kRowBytes <= k3BoxBytes, "layer-3 box");
-static_assert(k3Outputs % kEpiThreads == 0, "whole outputs per epilogue thread");
+static_assert(k3TmemCols == 128, "TMEM allocations are powers of two");
 static_assert(k3Smem <= 227 * 1024, "shared memory per CTA");
 
-// Named barrier 1 of the four epilogue warps (the non-aligned forms: lanes
-// may arrive apart); the OR reduction makes a give-up decision of any one
-// thread the decision of all, so they take the same barriers.
-__device__ __forceinline__ bool epi_any(bool pred)
-{
-    uint32_t r;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p, q;\n\t"
-        "setp.ne.u32 p, %1, 0;\n\t"
-        "barrier.red.or.pred q, 1, 128, p;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t"
-        "}\n"
-        : "=r"(r)
-        : "r"(pred ? 1u : 0u)
-        : "memory");
-    return r != 0;
-}
-
-__device__ __forceinline__ void epi_sync() { asm volatile("barrier.sync 1, 128;" ::: "memory"); }
-
 template <int kOut, bool kPair>
-__global__ void __launch_bounds__(kConvThreads, 1)
+__global__ void __launch_bounds__(k3Threads, 1)
     k_layer3_tc(const __grid_constant__ CUtensorMap in_map, ConvGrid g, const float* __restrict__ w3, float* out,
                 PermMap pm, int* status)
 {
@@ -624,8 +626,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* sA = smem;                                       // k3Stages x k3StageBytes
     unsigned char* sW = smem + k3Stages * k3StageBytes;             // + and - weight tiles
-    float* sD = (float*)(sW + 2 * k3WTileBytes);                    // k3Rows x k3DStride
-    uint64_t* full = (uint64_t*)(sD + k3Rows * k3DStride);
+    uint64_t* full = (uint64_t*)(sW + 2 * k3Tiles * k3Tile);
     uint64_t* empty = full + k3Stages;
     uint64_t* tfull = empty + k3Stages;
     uint64_t* tempty = tfull + 2;
@@ -634,20 +635,24 @@ __global__ void __launch_bounds__(kConvThreads, 1)
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    const int tx = (g.nx + k3X - 1) / k3X, ty = (g.ny + k3Y - 1) / k3Y, tz = (g.nz + k3Z - 1) / k3Z;
+    const int tx = (g.nx + kOX - 1) / kOX, ty = (g.ny + kTY - 1) / kTY, tz = (g.nz + kTZ - 1) / kTZ;
     const long per_sample = (long)tx * ty * tz;
     const long ntiles = per_sample * g.nb;
 
-    // weight tiles: row t = tap, 16 channels; the bf16 weight, halved and
-    // negated for the pair (exact in bf16)
-    for(int i = tid; i < k3N * kNetCh; i += kConvThreads)
+    // weight tile (dy, dz): column dx + 1 takes that tap, the others are zero
+    for(int i = tid; i < k3Tiles * k3PlaneCols * kNetCh; i += k3Threads)
     {
-        const int t = i / kNetCh, c = i % kNetCh;
-        float w = t < 27 ? __bfloat162float(__float2bfloat16_rn(w3[(t * kNetCh + c) * kNetCh])) : 0.f;
-        if(kPair) w *= 0.5f;
-        const uint32_t off = kmajor_off(t, c >> 3) + (uint32_t)(c & 7) * 2;
+        const int c = i % kNetCh, col = i / kNetCh % k3PlaneCols, tile = i / (kNetCh * k3PlaneCols);
+        float w = 0.f;
+        if(col < 3)
+        {
+            const int t = (2 - tile % 3) * 9 + tile / 3 * 3 + col;
+            w = __bfloat162float(__float2bfloat16_rn(w3[(t * kNetCh + c) * kNetCh]));
+            if(kPair) w *= 0.5f;  // exact in bf16
+        }
+        const uint32_t off = (uint32_t)(tile * k3Tile) + kmajor_off(col, c >> 3) + (uint32_t)(c & 7) * 2;
         *reinterpret_cast<__nv_bfloat16*>(sW + off) = __float2bfloat16_rn(w);
-        *reinterpret_cast<__nv_bfloat16*>(sW + k3WTileBytes + off) = __float2bfloat16_rn(-w);
+        *reinterpret_cast<__nv_bfloat16*>(sW + k3Tiles * k3Tile + off) = __float2bfloat16_rn(-w);
     }
     if(tid == 0)
     {
@@ -659,7 +664,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
         for(int a = 0; a < 2; ++a)
         {
             mbar_init(&tfull[a], 1);
-            mbar_init(&tempty[a], kEpiThreads);
+            mbar_init(&tempty[a], k3EpiThreads);
         }
         *abort_flag = 0;
     }
@@ -670,7 +675,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     tc_fence_after();
     const uint32_t tmem = *tholder;
     pdl_wait();  // from here on the previous kernel's output is read
-    constexpr uint32_t kBoxTx = (uint32_t)(k3Rows * kRowBytes) * (kPair ? 2u : 1u);
+    constexpr uint32_t kBoxTx = (uint32_t)kCopyBytes * (kPair ? 2u : 1u);
 
     if(warp == 0 && lane == 0)
     {
@@ -681,17 +686,12 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             const int st = (int)(issued % k3Stages);
             const uint32_t ph = (uint32_t)((issued / k3Stages) & 1);
             if(!role_wait(&empty[st], ph ^ 1u, abort_flag, status, 3)) break;
-            const int b = (int)(tile / per_sample);
-            long t2 = tile - (long)b * per_sample;
-            const int bz = (int)(t2 / ((long)tx * ty));
-            t2 -= (long)bz * tx * ty;
-            const int by = (int)(t2 / tx), bx = (int)(t2 - (long)by * tx);
+            const Brick bk = brick_of(g, tile, tx, ty, per_sample);
             mbar_expect_tx(&full[st], kBoxTx);
             unsigned char* dst = sA + st * k3StageBytes;
-            tma_load_5d(dst, &in_map, 0, bx * k3X - 1, by * k3Y - 1, bz * k3Z - 1, b, &full[st]);
+            tma_load_5d(dst, &in_map, 0, bk.x0 - 1, bk.y0 - 1, bk.z0 - 1, bk.b, &full[st]);
             if(kPair)
-                tma_load_5d(dst + k3BoxBytes, &in_map, 0, bx * k3X - 1, by * k3Y - 1, bz * k3Z - 1, b + g.nb,
-                            &full[st]);
+                tma_load_5d(dst + k3BoxBytes, &in_map, 0, bk.x0 - 1, bk.y0 - 1, bk.z0 - 1, bk.b + g.nb, &full[st]);
         }
         if(*abort_flag)
         {
@@ -703,9 +703,7 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     else if(warp == 1 && lane == 0)
     {
         // ---- MMA issuer
-        constexpr uint32_t idesc = umma_idesc_bf16(128, k3N, false, false);
-        const uint64_t bpos = umma_desc(smem_u32(sW), 128, 256);
-        const uint64_t bneg = umma_desc(smem_u32(sW + k3WTileBytes), 128, 256);
+        const uint64_t bd = umma_desc(smem_u32(sW), 128, 256);
         long i = 0;
         for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++i)
         {
@@ -718,12 +716,36 @@ __global__ void __launch_bounds__(kConvThreads, 1)
             tc_fence_after();
             const uint64_t a0 = umma_desc_sw32(smem_u32(sA + st * k3StageBytes));
             const uint32_t d0 = tmem + (uint32_t)(acc * k3AccCols);
+            // as in k_conv16: plane q feeds output planes mt in [lo, hi] with dz
+            // tile mt - q + 2, and first writes plane q by an MMA of its own
 #pragma unroll
-            for(int c = 0; c < k3Chunks; ++c)
+            for(int q = 0; q < kTZ + 2; ++q)
             {
-                const uint64_t ac = a0 + (uint64_t)((c * 128 * kRowBytes) >> 4);
-                mma_bf16(d0 + c * k3N, ac, bpos, idesc, 0u);
-                if(kPair) mma_bf16(d0 + c * k3N, ac + (uint64_t)(k3BoxBytes >> 4), bneg, idesc, 1u);
+                const int lo = q - 2 < 0 ? 0 : q - 2;
+                const int hi = q < kTZ - 1 ? q : kTZ - 1;
+#pragma unroll
+                for(int dyi = 0; dyi < 3; ++dyi)
+                {
+                    const uint64_t ad = a0 + (uint64_t)(((q * kHY + dyi) * kTX * kRowBytes) >> 4);
+                    auto mma = [&](int m0, int m1, uint32_t accumulate) {
+                        const uint32_t idesc = umma_idesc_bf16(128, (m1 - m0 + 1) * k3PlaneCols, false, false);
+                        const uint64_t bs = bd + (uint64_t)(((dyi * 3 + m0 - q + 2) * k3Tile) >> 4);
+                        const uint32_t d = d0 + (uint32_t)(m0 * k3PlaneCols);
+                        mma_bf16(d, ad, bs, idesc, accumulate);
+                        if(kPair)
+                            mma_bf16(d, ad + (uint64_t)(k3BoxBytes >> 4), bs + (uint64_t)((k3Tiles * k3Tile) >> 4),
+                                     idesc, 1u);
+                    };
+                    if(q <= kTZ - 1 && dyi == 0)
+                    {
+                        if(hi > lo) mma(lo, hi - 1, 1u);
+                        mma(hi, hi, 0u);
+                    }
+                    else
+                    {
+                        mma(lo, hi, 1u);
+                    }
+                }
             }
             mma_commit(&empty[st]);   // stage free once these MMAs have read it
             mma_commit(&tfull[acc]);  // accumulator ready for the epilogue
@@ -739,56 +761,36 @@ __global__ void __launch_bounds__(kConvThreads, 1)
     {
         // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31
         const int qd = warp & 3;
-        const int et = tid - 64;  // 0 .. 127
+        const int m = qd * 32 + lane;
         long i = 0;
         for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++i)
         {
             const int acc = (int)(i & 1);
             const uint32_t aph = (uint32_t)((i >> 1) & 1);
             const bool ok = role_wait(&tfull[acc], aph, abort_flag, status, 6);
-            if(epi_any(!ok)) break;
-            __syncwarp();  // tcgen05.ld is warp-collective
+            if(!__all_sync(0xffffffffu, ok)) break;  // tcgen05.ld is warp-collective
             tc_fence_after();
-#pragma unroll 1
-            for(int c = 0; c < k3Chunks; ++c)
-            {
-                float v[32];
-                const uint32_t ta = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(acc * k3AccCols + c * k3N);
-                tmem_ld16(ta, *reinterpret_cast<float(*)[16]>(v));
-                tmem_ld16(ta + 16, *reinterpret_cast<float(*)[16]>(v + 16));
-                const int row = c * 128 + qd * 32 + lane;
-                if(row < k3Rows)
-                {
-#pragma unroll
-                    for(int t = 0; t < 27; ++t) sD[row * k3DStride + t] = v[t];
-                }
-            }
+            float v[kTZ][4];
+            tmem_ld4x4(tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(acc * k3AccCols), k3PlaneCols, v);
             tc_fence_before();
             mbar_arrive(&tempty[acc]);  // the accumulator may take the next brick
-            epi_sync();                 // every staged point's taps are in shared memory
-            const int b = (int)(tile / per_sample);
-            long t2 = tile - (long)b * per_sample;
-            const int bz = (int)(t2 / ((long)tx * ty));
-            t2 -= (long)bz * tx * ty;
-            const int by = (int)(t2 / tx), bx = (int)(t2 - (long)by * tx);
+            const Brick bk = brick_of(g, tile, tx, ty, per_sample);
+            // row m is staged point (xi, yi) of a plane; xi = 0 and kTX - 1 are the halo columns
+            const int xi = m % kTX;
+            const int x = bk.x0 - 1 + xi, y = bk.y0 + m / kTX;
+            const bool halo = xi == 0 || xi == kTX - 1;
 #pragma unroll
-            for(int k = 0; k < k3Outputs / kEpiThreads; ++k)
+            for(int mt = 0; mt < kTZ; ++mt)
             {
-                const int o = et + k * kEpiThreads;
-                const int ox = o % k3X, oy = (o / k3X) % k3Y, oz = o / (k3X * k3Y);
-                const int x = bx * k3X + ox, y = by * k3Y + oy, z = bz * k3Z + oz;
-                if(x >= g.nx || y >= g.ny || z >= g.nz) continue;
-                float sum = 0.f;
-#pragma unroll
-                for(int t = 0; t < 27; ++t)
-                {
-                    const int dz = t / 9 - 1, dy = (t / 3) % 3 - 1, dx = t % 3 - 1;
-                    const int r = ((oz + 1 + dz) * k3HY + (oy + 1 + dy)) * k3HX + (ox + 1 + dx);
-                    sum += sD[r * k3DStride + t];
-                }
+                // out(x) = D_{dx=-1}[x - 1] + D_{dx=0}[x] + D_{dx=+1}[x + 1]
+                const float left = __shfl_up_sync(0xffffffffu, v[mt][0], 1);
+                const float right = __shfl_down_sync(0xffffffffu, v[mt][2], 1);
+                const float sum = (left + v[mt][1]) + right;
+                const int z = bk.z0 + mt;
+                if(halo || x >= g.nx || y >= g.ny || z >= g.nz) continue;
                 if constexpr(kOut == 2)
                 {
-                    out[(((long)b * g.nz + z) * g.ny + y) * g.nx + x] = sum;
+                    out[(((long)bk.b * g.nz + z) * g.ny + y) * g.nx + x] = sum;
                 }
                 else
                 {
@@ -797,7 +799,6 @@ __global__ void __launch_bounds__(kConvThreads, 1)
                     else *xo = sum;
                 }
             }
-            epi_sync();  // shared memory free for the next brick
         }
     }
     tc_fence_before();
@@ -988,16 +989,18 @@ __global__ void __launch_bounds__(kWgThreads) k_conv16_wgrad(ConvGrid g, const _
                 tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(t * kWgN + r * kNetCh), v);
                 if(yy < kWgLinesA && dy >= -1 && dy <= 1)
                 {
-                    float* d = sums + ((t / 3 * 9 + (dy + 1) * 3 + t % 3) * kNetCh + ci) * kNetCh;
+                    // [tap][co][ci]: the lanes of a line on consecutive words
+                    float* d = sums + (t / 3 * 9 + (dy + 1) * 3 + t % 3) * kNetCh * kNetCh + ci;
 #pragma unroll
-                    for(int c = 0; c < 16; ++c) d[c] += v[c];
+                    for(int c = 0; c < 16; ++c) d[c * kNetCh] += v[c];
                 }
             }
         }
         __syncthreads();
     }
     float* dst = partial + (size_t)blockIdx.x * kNetLayerWeights;
-    for(int i = tid; i < kNetLayerWeights; i += kWgThreads) dst[i] = ok ? sums[i] : 0.f;
+    for(int i = tid; i < kNetLayerWeights; i += kWgThreads)
+        dst[i] = ok ? sums[(i & ~255) | ((i & 15) << 4) | ((i >> 4) & 15)] : 0.f;
     tc_fence_before();
     __syncthreads();
     if(warp == 0) tmem_free(tmem, 512);
@@ -1603,11 +1606,12 @@ static int layer3_launch(const ConvGrid& g, const void* a2, const float* w3, flo
     }
     CUtensorMap map;
     const ConvGrid gin{kPair ? 2 * g.nb : g.nb, g.nz, g.ny, g.nx};
-    HB_RETURN_IF(bf16_box_map(gin, a2, k3HX, k3HY, k3HZ, &map));
-    const long tiles = (long)g.nb * ((g.nx + k3X - 1) / k3X) * ((g.ny + k3Y - 1) / k3Y) * ((g.nz + k3Z - 1) / k3Z);
+    HB_RETURN_IF(bf16_box_map(gin, a2, kTX, kHY, kHZ, &map));
+    const long tiles =
+        (long)g.nb * ((g.nx + kOX - 1) / kOX) * ((g.ny + kTY - 1) / kTY) * ((g.nz + kTZ - 1) / kTZ);
     const long cap = sm_count();
     const int grid = (int)(tiles < cap ? tiles : cap);
-    HB_CUDA(launch_pdl_net(k_layer3_tc<kOut, kPair>, dim3(grid), dim3(kConvThreads), (size_t)k3Smem, s, map, g, w3,
+    HB_CUDA(launch_pdl_net(k_layer3_tc<kOut, kPair>, dim3(grid), dim3(k3Threads), (size_t)k3Smem, s, map, g, w3,
                            out, pm, status));
     return 0;
 }
