@@ -85,6 +85,21 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
+// One lane of the (converged) warp.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .b32 r;\n\t"
+        "elect.sync r|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ void mma_commit(uint64_t* mbar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(mbar))
@@ -821,9 +836,11 @@ __global__ void __launch_bounds__(k3Threads, 1)
 // for one (dz, dx): the plane and the start x of A.  The nine (dz, dx)
 // accumulators take 432 TMEM columns; the (line, line) pairs one apart are
 // the dy taps, summed at the end.  A CTA walks units of 3 lines x 16 x x 8
-// planes, the next unit's loads in flight while the MMAs of this one run.  A
-// training batch of 64 samples of 16^3 (three weight gradients): 1572 -> 392 us
-// with the masked epilogue's prefetch above.
+// planes: eight warps fetch units into a ring of three stages, a ninth issues the
+// MMAs from one elected lane (72 a unit, 40 cycles each; issued by a loader thread
+// between two block barriers they took 53, and loads and MMAs met at each unit).
+// A training batch of 64 samples of 16^3 (three weight gradients, two
+// convolutions): im2col 1572 us, bricks 361, with the warps' split 299.
 constexpr int kWgX = 16, kWgLines = 3, kWgZ = 8;                  // gradient points of a unit
 constexpr int kWgXA = kWgX + 2, kWgLinesA = kWgLines + 2, kWgZA = kWgZ + 2;  // input points, with the halo
 constexpr int kWgRowA = kWgXA * 16, kWgRowB = kWgX * 16;          // bytes of one line of one half
@@ -831,11 +848,12 @@ constexpr int kWgPlaneA = kWgLinesA * 2 * kWgRowA, kWgPlaneB = kWgLines * 2 * kW
 constexpr int kWgN = kWgLines * kNetCh;                           // 48 columns per (dz, dx)
 constexpr int kWgOffB = kWgZA * kWgPlaneA;
 constexpr int kWgStage = kWgOffB + kWgZ * kWgPlaneB;
-constexpr int kWgThreads = 256;
+constexpr int kWgThreads = 256;                                   // loaders (and one warp that issues the MMAs)
 constexpr int kWgItemsA = kWgZA * kWgLinesA * kWgXA * 2, kWgItemsB = kWgZ * kWgLines * kWgX * 2;  // 16 B each
 constexpr int kWgLoadsA = (kWgItemsA + kWgThreads - 1) / kWgThreads;
 constexpr int kWgLoadsB = (kWgItemsB + kWgThreads - 1) / kWgThreads;
-constexpr int kWgSmem = 2 * kWgStage + 128;
+constexpr int kWgStages = 3;
+constexpr int kWgSmem = kWgStages * kWgStage + 128;
 static_assert(9 * kWgN <= 512 && kWgStage % 128 == 0, "accumulators and stages");
 // the last plane's A operand reads 16 halves and two 8-point groups from its start
 static_assert((kWgZA - 1) * kWgPlaneA + 15 * kWgRowA + 256 + 32 <= kWgStage, "A reads stay in the stage");
@@ -853,14 +871,16 @@ __host__ __device__ inline WgUnits wg_units(const ConvGrid& g)
     return WgUnits{tx, ty, tz, (long)g.nb * tz * ty * tx};
 }
 
-__global__ void __launch_bounds__(kWgThreads) k_conv16_wgrad(ConvGrid g, const __nv_bfloat16* __restrict__ x,
-                                                             const __nv_bfloat16* __restrict__ gr,
-                                                             float* __restrict__ partial, int* status)
+__global__ void __launch_bounds__(kWgThreads + 32, 1)
+    k_conv16_wgrad(ConvGrid g, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gr,
+                   float* __restrict__ partial, int* status)
 {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
-    __shared__ uint64_t mbar[2];
+    __shared__ uint64_t full[kWgStages], empty[kWgStages], finished;
     __shared__ uint32_t tholder;
+    __shared__ int gave_up;
+    volatile int* abort_flag = &gave_up;
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
@@ -868,115 +888,120 @@ __global__ void __launch_bounds__(kWgThreads) k_conv16_wgrad(ConvGrid g, const _
 
     if(tid == 0)
     {
-        mbar_init(&mbar[0], 1);
-        mbar_init(&mbar[1], 1);
+        for(int k = 0; k < kWgStages; ++k)
+        {
+            mbar_init(&full[k], kWgThreads);
+            mbar_init(&empty[k], 1);
+        }
+        mbar_init(&finished, 1);
+        gave_up = 0;
     }
     if(warp == 0) tmem_alloc(&tholder, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tholder;
-    constexpr uint32_t idesc = umma_idesc_bf16(128, kWgN, true, true);
 
-    // 16-byte items of unit u: (plane, line, x, half), zero outside the sample
-    uint4 va[kWgLoadsA], vb[kWgLoadsB];
-    auto load = [&](long u) {
-        const int bx = (int)(u % U.tx);
-        const long q1 = u / U.tx;
-        const int by = (int)(q1 % U.ty);
-        const long q2 = q1 / U.ty;
-        const int bz = (int)(q2 % U.tz);
-        const long b = q2 / U.tz;
-        const int x0 = bx * kWgX, y0 = by * kWgLines, z0 = bz * kWgZ;
-        auto fetch = [&](const __nv_bfloat16* src, int z, int y, int xx, int half) {
-            if((unsigned)z >= (unsigned)g.nz || (unsigned)y >= (unsigned)g.ny || (unsigned)xx >= (unsigned)g.nx)
-                return make_uint4(0, 0, 0, 0);
-            return __ldg(reinterpret_cast<const uint4*>(src + (((b * g.nz + z) * g.ny + y) * g.nx + xx) * kNetCh) +
-                         half);
+    if(tid < kWgThreads)
+    {
+        // ---- loaders: 16-byte items of unit u (plane, line, x, half), zero outside the sample
+        uint4 va[kWgLoadsA], vb[kWgLoadsB];
+        auto load = [&](long u) {
+            const int bx = (int)(u % U.tx);
+            const long q1 = u / U.tx;
+            const int by = (int)(q1 % U.ty);
+            const long q2 = q1 / U.ty;
+            const int bz = (int)(q2 % U.tz);
+            const long b = q2 / U.tz;
+            const int x0 = bx * kWgX, y0 = by * kWgLines, z0 = bz * kWgZ;
+            auto fetch = [&](const __nv_bfloat16* src, int z, int y, int xx, int half) {
+                if((unsigned)z >= (unsigned)g.nz || (unsigned)y >= (unsigned)g.ny || (unsigned)xx >= (unsigned)g.nx)
+                    return make_uint4(0, 0, 0, 0);
+                return __ldg(
+                    reinterpret_cast<const uint4*>(src + (((b * g.nz + z) * g.ny + y) * g.nx + xx) * kNetCh) + half);
+            };
+#pragma unroll
+            for(int k = 0; k < kWgLoadsA; ++k)
+            {
+                const int i = tid + k * kWgThreads, q = i >> 1, line = q / kWgXA;
+                va[k] = i < kWgItemsA ? fetch(x, z0 - 1 + line / kWgLinesA, y0 - 1 + line % kWgLinesA,
+                                              x0 - 1 + q % kWgXA, i & 1)
+                                      : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for(int k = 0; k < kWgLoadsB; ++k)
+            {
+                const int i = tid + k * kWgThreads, q = i >> 1, line = q / kWgX;
+                vb[k] = i < kWgItemsB ? fetch(gr, z0 + line / kWgLines, y0 + line % kWgLines, x0 + q % kWgX, i & 1)
+                                      : make_uint4(0, 0, 0, 0);
+            }
         };
-#pragma unroll
-        for(int k = 0; k < kWgLoadsA; ++k)
+        load(blockIdx.x);
+        int k = 0;
+        for(long u = blockIdx.x; u < U.count; u += gridDim.x, ++k)
         {
-            const int i = tid + k * kWgThreads, q = i >> 1, line = q / kWgXA;
-            va[k] = i < kWgItemsA ? fetch(x, z0 - 1 + line / kWgLinesA, y0 - 1 + line % kWgLinesA,
-                                          x0 - 1 + q % kWgXA, i & 1)
-                                  : make_uint4(0, 0, 0, 0);
-        }
+            const int st = k % kWgStages;
+            // the MMAs that read this stage kWgStages units ago
+            if(!role_wait(&empty[st], (uint32_t)((k / kWgStages) & 1) ^ 1u, abort_flag, status, 2)) break;
+            unsigned char* sA = smem + st * kWgStage;
 #pragma unroll
-        for(int k = 0; k < kWgLoadsB; ++k)
-        {
-            const int i = tid + k * kWgThreads, q = i >> 1, line = q / kWgX;
-            vb[k] = i < kWgItemsB ? fetch(gr, z0 + line / kWgLines, y0 + line % kWgLines, x0 + q % kWgX, i & 1)
-                                  : make_uint4(0, 0, 0, 0);
+            for(int j = 0; j < kWgLoadsA; ++j)
+            {
+                const int i = tid + j * kWgThreads, q = i >> 1, line = q / kWgXA;
+                if(i < kWgItemsA)
+                    *reinterpret_cast<uint4*>(sA + (line * 2 + (i & 1)) * kWgRowA + q % kWgXA * 16) = va[j];
+            }
+#pragma unroll
+            for(int j = 0; j < kWgLoadsB; ++j)
+            {
+                const int i = tid + j * kWgThreads, q = i >> 1, line = q / kWgX;
+                if(i < kWgItemsB)
+                    *reinterpret_cast<uint4*>(sA + kWgOffB + (line * 2 + (i & 1)) * kWgRowB + q % kWgX * 16) = vb[j];
+            }
+            fence_async_smem();
+            mbar_arrive(&full[st]);
+            if(u + gridDim.x < U.count) load(u + gridDim.x);
         }
-    };
-
-    uint32_t phase[2] = {0, 0};
-    bool ok = true;
-    int done = 0;  // units whose MMAs were issued
-    load(blockIdx.x);
-    for(long u = blockIdx.x; u < U.count; u += gridDim.x, ++done)
+    }
+    else
     {
-        const int st = done & 1;
-        unsigned char* sA = smem + st * kWgStage;
-        bool arrived = true;
-        if(done >= 2)  // the MMAs that read this stage two units ago
+        // ---- MMA issuer: the whole warp walks the loop, one elected lane issues
+        constexpr uint32_t idesc = umma_idesc_bf16(128, kWgN, true, true);
+        int k = 0;
+        for(long u = blockIdx.x; u < U.count; u += gridDim.x, ++k)
         {
-            arrived = mbar_wait(&mbar[st], phase[st]);
-            phase[st] ^= 1u;
-        }
-        if(__syncthreads_and(arrived) == 0)
-        {
-            ok = false;
-            phase[st] ^= 1u;  // waited for once more below
-            break;
-        }
-#pragma unroll
-        for(int k = 0; k < kWgLoadsA; ++k)
-        {
-            const int i = tid + k * kWgThreads, q = i >> 1, line = q / kWgXA;
-            if(i < kWgItemsA)
-                *reinterpret_cast<uint4*>(sA + (line * 2 + (i & 1)) * kWgRowA + q % kWgXA * 16) = va[k];
-        }
-#pragma unroll
-        for(int k = 0; k < kWgLoadsB; ++k)
-        {
-            const int i = tid + k * kWgThreads, q = i >> 1, line = q / kWgX;
-            if(i < kWgItemsB)
-                *reinterpret_cast<uint4*>(sA + kWgOffB + (line * 2 + (i & 1)) * kWgRowB + q % kWgX * 16) = vb[k];
-        }
-        fence_async_smem();
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
-        if(tid == 0)
-        {
-            const uint64_t ad = umma_desc(smem_u32(sA), 128, kWgRowA);
-            const uint64_t bd = umma_desc(smem_u32(sA + kWgOffB), 128, kWgRowB);
+            const int st = k % kWgStages;
+            const bool there = role_wait(&full[st], (uint32_t)((k / kWgStages) & 1), abort_flag, status, 2);
+            if(!__all_sync(0xffffffffu, there)) break;
+            tc_fence_after();
+            const uint64_t ad = umma_desc(smem_u32(smem + st * kWgStage), 128, kWgRowA);
+            const uint64_t bd = umma_desc(smem_u32(smem + st * kWgStage + kWgOffB), 128, kWgRowB);
+            if(elect_one())
+            {
 #pragma unroll 1
-            for(int z = 0; z < kWgZ; ++z)
+                for(int z = 0; z < kWgZ; ++z)
 #pragma unroll
-                for(int t = 0; t < 9; ++t)
-                    mma_bf16(tmem + (uint32_t)(t * kWgN), ad + (uint64_t)(((z + t / 3) * kWgPlaneA + t % 3 * 16) >> 4),
-                             bd + (uint64_t)((z * kWgPlaneB) >> 4), idesc, (done == 0 && z == 0) ? 0u : 1u);
-            mma_commit(&mbar[st]);
+                    for(int t = 0; t < 9; ++t)
+                        mma_bf16(tmem + (uint32_t)(t * kWgN),
+                                 ad + (uint64_t)(((z + t / 3) * kWgPlaneA + t % 3 * 16) >> 4),
+                                 bd + (uint64_t)((z * kWgPlaneB) >> 4), idesc, (k == 0 && z == 0) ? 0u : 1u);
+                mma_commit(&empty[st]);
+            }
+            __syncwarp();
         }
+        // every MMA issued (also after a time-out: they finish before the CTA leaves)
+        if(elect_one()) mma_commit(&finished);
         __syncwarp();
-        if(u + gridDim.x < U.count) load(u + gridDim.x);
     }
-    // every unit's MMAs (also after a time-out: they finish before the CTA leaves)
-    for(int k = max(0, done - 2); k < done; ++k)
-    {
-        const bool arrived = mbar_wait(&mbar[k & 1], phase[k & 1]);
-        phase[k & 1] ^= 1u;
-        if(__syncthreads_and(arrived) == 0) ok = false;
-    }
+    if(!mbar_wait(&finished, 0)) *abort_flag = 1;
+    __syncthreads();
+    const bool ok = *abort_flag == 0;
     if(!ok && tid == 0) atomicExch(status, 2);
     tc_fence_after();
 
     // accumulator row = (input line yy, channel), column group r = gradient line: dy = yy - 1 - r
     float* sums = reinterpret_cast<float*>(smem);
-    for(int i = tid; i < kNetLayerWeights; i += kWgThreads) sums[i] = 0.f;
+    for(int i = tid; i < kNetLayerWeights; i += blockDim.x) sums[i] = 0.f;
     __syncthreads();
     for(int r = 0; r < kWgLines; ++r)
     {
@@ -999,7 +1024,7 @@ __global__ void __launch_bounds__(kWgThreads) k_conv16_wgrad(ConvGrid g, const _
         __syncthreads();
     }
     float* dst = partial + (size_t)blockIdx.x * kNetLayerWeights;
-    for(int i = tid; i < kNetLayerWeights; i += kWgThreads)
+    for(int i = tid; i < kNetLayerWeights; i += blockDim.x)
         dst[i] = ok ? sums[(i & ~255) | ((i & 15) << 4) | ((i >> 4) & 15)] : 0.f;
     tc_fence_before();
     __syncthreads();
@@ -1653,7 +1678,7 @@ int launch_conv16_wgrad(const ConvGrid& g, const void* x, const void* gr, float*
     const long units = wg_units(g).count;
     const int most = conv16_wgrad_parts(g.points());
     const int parts = (int)(units < most ? units : most);
-    k_conv16_wgrad<<<parts, kWgThreads, kWgSmem, s>>>(g, (const __nv_bfloat16*)x, (const __nv_bfloat16*)gr, partial,
+    k_conv16_wgrad<<<parts, kWgThreads + 32, kWgSmem, s>>>(g, (const __nv_bfloat16*)x, (const __nv_bfloat16*)gr, partial,
                                                       status);
     HB_LAUNCHED();
     k_wgrad_reduce<<<kNetLayerWeights / 32, 256, 0, s>>>(parts, partial, dw);
