@@ -165,6 +165,37 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
     for(int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 48 consecutive columns: issued here, there after tmem_wait48.
+__device__ __forceinline__ void tmem_ld48(uint32_t taddr, uint32_t (&r)[48])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]),
+          "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47])
+        : "r"(taddr + 32));
+}
+
+// the values as operands: nothing that uses them moves above the wait
+__device__ __forceinline__ void tmem_wait48(uint32_t (&r)[48])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
+                   "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]),
+                   "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]),
+                   "+r"(r[29]), "+r"(r[30]), "+r"(r[31]), "+r"(r[32]), "+r"(r[33]), "+r"(r[34]), "+r"(r[35]),
+                   "+r"(r[36]), "+r"(r[37]), "+r"(r[38]), "+r"(r[39]), "+r"(r[40]), "+r"(r[41]), "+r"(r[42]),
+                   "+r"(r[43]), "+r"(r[44]), "+r"(r[45]), "+r"(r[46]), "+r"(r[47])::"memory");
+}
+
 // Four groups of four columns, `stride` columns apart.
 __device__ __forceinline__ void tmem_ld4x4(uint32_t taddr, uint32_t stride, float (&v)[4][4])
 {
@@ -246,6 +277,10 @@ __host__ __device__ constexpr int weight_slot(int t) { return ((t / 3) % 3) * 9 
 //               combination, ReLU / mask / permuted scatter, global stores
 //               (eight warps instead of four: a training batch, whose masked
 //               passes read the activations too, 371 -> 361 us).
+// Two samples of 128^3 took 96 us; with a sixth of the box rows loaded 94, a
+// third of the MMAs 76, no stores 92: latencies on the roles' paths, not a unit,
+// were the bound.  Carried brick coordinates, an elected issuer lane and one
+// tcgen05.ld wait a plane with the next plane's columns in flight: 81 us.
 // Stage and accumulator hand-offs are mbarriers (TMA complete_tx, MMA commit,
 // epilogue arrivals), so loads, MMAs and stores of consecutive bricks overlap.
 
@@ -287,19 +322,50 @@ struct Brick
     int b, x0, y0, z0;
 };
 
-__device__ __forceinline__ Brick brick_of(const ConvGrid& g, long tile, int tx, int ty, long per_sample)
+// The bricks of a CTA: tile, tile + step, ... with x fastest.  Their coordinates
+// are carried along (the divisions of a 64-bit tile number, done by every role for
+// every brick, were on each role's path).
+struct BrickWalk
 {
-    Brick r;
-    r.b = (int)(tile / per_sample);
-    long t2 = tile - (long)r.b * per_sample;
-    const int bz = (int)(t2 / ((long)tx * ty));
-    t2 -= (long)bz * tx * ty;
-    const int by = (int)(t2 / tx), bx = (int)(t2 - (long)by * tx);
-    r.x0 = bx * kOX;  // first output x; the box starts one point before
-    r.y0 = by * kTY;
-    r.z0 = bz * kTZ;
-    return r;
-}
+    int tx, ty, tz;          // bricks per axis
+    int b, bz, by, bx;       // the current one
+    int sb, sz, sy, sx;      // the step
+
+    __device__ BrickWalk(const ConvGrid& g, int ox, int oy, int oz, long tile, long step)
+        : tx((g.nx + ox - 1) / ox), ty((g.ny + oy - 1) / oy), tz((g.nz + oz - 1) / oz)
+    {
+        split(tile, b, bz, by, bx);
+        split(step, sb, sz, sy, sx);
+    }
+
+    __device__ void split(long t, int& tb, int& tbz, int& tby, int& tbx) const
+    {
+        const long q1 = t / tx, q2 = q1 / ty;
+        tbx = (int)(t - q1 * tx);
+        tby = (int)(q1 - q2 * ty);
+        tb = (int)(q2 / tz);
+        tbz = (int)(q2 - (long)tb * tz);
+    }
+
+    __device__ long count(int nb) const { return (long)tx * ty * tz * nb; }
+
+    __device__ __forceinline__ void next()
+    {
+        bx += sx;
+        int carry = bx >= tx;
+        bx -= carry ? tx : 0;
+        by += sy + carry;
+        carry = by >= ty;
+        by -= carry ? ty : 0;
+        bz += sz + carry;
+        carry = bz >= tz;
+        bz -= carry ? tz : 0;
+        b += sb + carry;
+    }
+
+    // first output point
+    __device__ __forceinline__ Brick at(int ox, int oy, int oz) const { return Brick{b, bx * ox, by * oy, bz * oz}; }
+};
 
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* mbar, uint32_t bytes)
 {
@@ -367,9 +433,8 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    const int tx = (g.nx + kOX - 1) / kOX, ty = (g.ny + kTY - 1) / kTY, tz = (g.nz + kTZ - 1) / kTZ;
-    const long per_sample = (long)tx * ty * tz;
-    const long ntiles = per_sample * g.nb;
+    BrickWalk walk(g, kOX, kTY, kTZ, blockIdx.x, gridDim.x);
+    const long ntiles = walk.count(g.nb);
 
     for(int i = tid; i < kNetWeightTileBytes / 16; i += kConvThreads)
         reinterpret_cast<uint4*>(sW)[i] = reinterpret_cast<const uint4*>(wB)[i];
@@ -399,12 +464,12 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
     {
         // ---- TMA producer
         long issued = 0;
-        for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++issued)
+        for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, walk.next(), ++issued)
         {
             const int st = (int)(issued % kStages);
             const uint32_t ph = (uint32_t)((issued / kStages) & 1);
             if(!role_wait(&empty[st], ph ^ 1u, abort_flag, status, 3)) break;
-            const Brick bk = brick_of(g, tile, tx, ty, per_sample);
+            const Brick bk = walk.at(kOX, kTY, kTZ);
             mbar_expect_tx(&full[st], (uint32_t)kCopyBytes);
             tma_load_5d(sA + st * kStageBytes, &in_map, 0, bk.x0 - 1, bk.y0 - 1, bk.z0 - 1, bk.b, &full[st]);
         }
@@ -412,22 +477,12 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
         {
             // let the loads already issued land before the CTA's shared memory goes away
             for(long k = issued - kStages < 0 ? 0 : issued - kStages; k < issued; ++k)
-            {
-                uint32_t done = 0;
-                const uint32_t a = smem_u32(&full[k % kStages]);
-                for(uint32_t i = 0; i < kSpinLimit && !done; ++i)
-                    asm volatile(
-                        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                        "selp.u32 %0, 1, 0, p;\n\t}\n"
-                        : "=r"(done)
-                        : "r"(a), "r"((uint32_t)((k / kStages) & 1))
-                        : "memory");
-            }
+                mbar_wait(&full[k % kStages], (uint32_t)((k / kStages) & 1));
         }
     }
-    else if(warp == 1 && lane == 0)
+    else if(warp == 1)
     {
-        // ---- MMA issuer
+        // ---- MMA issuer: the whole warp walks the loop, one elected lane issues
         const uint64_t bd0 = umma_desc(smem_u32(sW), 128, 256);
         long i = 0;
         for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++i)
@@ -436,8 +491,9 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
             const uint32_t ph = (uint32_t)((i / kStages) & 1);
             const int acc = (int)(i & 1);
             const uint32_t aph = (uint32_t)((i >> 1) & 1);
-            if(!role_wait(&tempty[acc], aph ^ 1u, abort_flag, status, 4)) break;
-            if(!role_wait(&full[st], ph, abort_flag, status, 5)) break;
+            const bool ready = role_wait(&tempty[acc], aph ^ 1u, abort_flag, status, 4) &&
+                               role_wait(&full[st], ph, abort_flag, status, 5);
+            if(!__all_sync(0xffffffffu, ready)) break;
             tc_fence_after();
             // descriptors = base + compile-time offset (the 14-bit start field
             // holds address / 16 and stays below 2^14 for any smem address)
@@ -447,49 +503,45 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
             // in [lo, hi]; output plane mt takes dz block j = mt - q + 2 of the
             // row shift's 144-row operand.  Output plane q is first written at
             // (q, dy = -1), with the accumulate flag off, by an MMA of its own.
-#pragma unroll
-            for(int q = 0; q < kTZ + 2; ++q)
+            if(elect_one())
             {
-                const int lo = q - 2 < 0 ? 0 : q - 2;
-                const int hi = q < kTZ - 1 ? q : kTZ - 1;
 #pragma unroll
-                for(int dyi = 0; dyi < 3; ++dyi)
+                for(int q = 0; q < kTZ + 2; ++q)
                 {
-                    const int row0 = (q * kHY + dyi) * kTX;
-                    const uint64_t ad = ad0 + (uint64_t)((row0 * kRowBytes) >> 4);
-                    const uint64_t bs = bd0 + (uint64_t)((dyi * 9 * 512) >> 4);
-                    auto mma = [&](int m0, int m1, uint32_t accumulate) {
-                        const uint32_t idesc = umma_idesc_bf16(128, (m1 - m0 + 1) * kPlaneCols, false, false);
-                        mma_bf16(d0 + m0 * kPlaneCols, ad, bs + (uint64_t)(((m0 - q + 2) * 3 * 512) >> 4), idesc,
-                                 accumulate);
-                    };
-                    if(q <= kTZ - 1 && dyi == 0)
+                    const int lo = q - 2 < 0 ? 0 : q - 2;
+                    const int hi = q < kTZ - 1 ? q : kTZ - 1;
+#pragma unroll
+                    for(int dyi = 0; dyi < 3; ++dyi)
                     {
-                        if(hi > lo) mma(lo, hi - 1, 1u);
-                        mma(hi, hi, 0u);
-                    }
-                    else
-                    {
-                        mma(lo, hi, 1u);
+                        const int row0 = (q * kHY + dyi) * kTX;
+                        const uint64_t ad = ad0 + (uint64_t)((row0 * kRowBytes) >> 4);
+                        const uint64_t bs = bd0 + (uint64_t)((dyi * 9 * 512) >> 4);
+                        auto mma = [&](int m0, int m1, uint32_t accumulate) {
+                            const uint32_t idesc = umma_idesc_bf16(128, (m1 - m0 + 1) * kPlaneCols, false, false);
+                            mma_bf16(d0 + m0 * kPlaneCols, ad, bs + (uint64_t)(((m0 - q + 2) * 3 * 512) >> 4), idesc,
+                                     accumulate);
+                        };
+                        if(q <= kTZ - 1 && dyi == 0)
+                        {
+                            if(hi > lo) mma(lo, hi - 1, 1u);
+                            mma(hi, hi, 0u);
+                        }
+                        else
+                        {
+                            mma(lo, hi, 1u);
+                        }
                     }
                 }
+                mma_commit(&empty[st]);   // stage free once these MMAs have read it
+                mma_commit(&tfull[acc]);  // accumulator ready for the epilogue
             }
-            mma_commit(&empty[st]);   // stage free once these MMAs have read it
-            mma_commit(&tfull[acc]);  // accumulator ready for the epilogue
+            __syncwarp();
         }
         if(*abort_flag && i > 0)
         {
             // MMAs in flight must finish before TMEM is released
             const long k = i - 1;
-            uint32_t done = 0;
-            const uint32_t a = smem_u32(&tfull[k & 1]);
-            for(uint32_t j = 0; j < kSpinLimit && !done; ++j)
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                    "selp.u32 %0, 1, 0, p;\n\t}\n"
-                    : "=r"(done)
-                    : "r"(a), "r"((uint32_t)((k >> 1) & 1))
-                    : "memory");
+            mbar_wait(&tfull[k & 1], (uint32_t)((k >> 1) & 1));
         }
     }
     else if(warp >= 2)
@@ -498,13 +550,14 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
         const int qd = warp & 3;
         const int m = qd * 32 + lane;
         constexpr int kPlanes = kTZ / 2;
+        static_assert(kPlanes == 2 && kPlaneCols == 48, "two planes a warp");
         const int mt0 = (warp - 2) / 4 * kPlanes;  // this warp's output planes of a brick
         long i = 0;
-        for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++i)
+        for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, walk.next(), ++i)
         {
             const int acc = (int)(i & 1);
             const uint32_t aph = (uint32_t)((i >> 1) & 1);
-            const Brick bk = brick_of(g, tile, tx, ty, per_sample);
+            const Brick bk = walk.at(kOX, kTY, kTZ);
             // row m is staged point (xi, yi) of the plane; xi = 0 and kTX - 1
             // are the halo columns
             const int xi = m % kTX;
@@ -528,28 +581,22 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
                     mask[2 * mt + 1] = __ldg(ap + 1);
                 }
             }
-            if(!role_wait(&tfull[acc], aph, abort_flag, status, 6)) break;
+            const bool ok = role_wait(&tfull[acc], aph, abort_flag, status, 6);
+            if(!__all_sync(0xffffffffu, ok)) break;  // tcgen05.ld is warp-collective
             tc_fence_after();
-#pragma unroll(kOut == kOutMaskBf16 ? kPlanes : 1)
-            for(int mt = 0; mt < kPlanes; ++mt)
-            {
-                // out(x) = D_{dx=-1}[x - 1] + D_{dx=0}[x] + D_{dx=+1}[x + 1]: rows
-                // x +- 1 are the neighbouring lanes of the same 16-lane line
-                float dm[16], dc[16], dp[16], v[16];
-                const uint32_t ta =
-                    tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(acc * kAccCols + (mt0 + mt) * kPlaneCols);
-                tmem_ld16(ta, dm);
-                tmem_ld16(ta + kNetCh, dc);
-                tmem_ld16(ta + 2 * kNetCh, dp);
+            // out(x) = D_{dx=-1}[x - 1] + D_{dx=0}[x] + D_{dx=+1}[x + 1]: rows
+            // x +- 1 are the neighbouring lanes of the same 16-lane line
+            auto finish = [&](int mt, const uint32_t (&d)[48]) {
+                float v[16];
 #pragma unroll
                 for(int c = 0; c < 16; ++c)
                 {
-                    const float left = __shfl_up_sync(0xffffffffu, dm[c], 1);
-                    const float right = __shfl_down_sync(0xffffffffu, dp[c], 1);
-                    v[c] = (left + dc[c]) + right;
+                    const float left = __shfl_up_sync(0xffffffffu, __uint_as_float(d[c]), 1);
+                    const float right = __shfl_down_sync(0xffffffffu, __uint_as_float(d[32 + c]), 1);
+                    v[c] = (left + __uint_as_float(d[16 + c])) + right;
                 }
                 const int z = bk.z0 + mt0 + mt;
-                if(halo || x >= g.nx || y >= g.ny || z >= g.nz) continue;
+                if(halo || x >= g.nx || y >= g.ny || z >= g.nz) return;
                 const long p = (((long)bk.b * g.nz + z) * g.ny + y) * g.nx + x;
                 if constexpr(kOut == kOutReluBf16 || kOut == kOutMaskBf16)
                 {
@@ -587,9 +634,19 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
                     if constexpr(kOut == kOutPermSet) *xo = v[0];
                     else *xo += v[0];
                 }
-            }
+            };
+            // the second plane's columns on their way while the first is finished
+            const uint32_t ta = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(acc * kAccCols + mt0 * kPlaneCols);
+            uint32_t d0[48], d1[48];
+            tmem_ld48(ta, d0);
+            tmem_wait48(d0);
+            tmem_ld48(ta + kPlaneCols, d1);
+            finish(0, d0);
+            __syncwarp();
+            tmem_wait48(d1);
             tc_fence_before();
-            mbar_arrive(&tempty[acc]);
+            mbar_arrive(&tempty[acc]);  // the accumulator may take the next brick
+            finish(1, d1);
         }
     }
     tc_fence_before();
@@ -610,8 +667,8 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
 // (y(r) - y(-r)) / 2.  The epilogue is one small tcgen05.ld and two lane shuffles
 // per output plane.  (All 27 taps in N with the sums gathered from shared
 // memory, 27 floats a staged point, was bound by that gather: 120 us on an odd
-// 128^3 sample; this form takes about 75, the boxes' 32-byte rows now the bound.
-// The whole network there: 301 -> 252 us; 256^3 learned V-cycle 661 -> 651 us.)
+// 128^3 sample; this form takes 52, of it 42 MMAs a brick about 30.  The whole
+// network there: 301 -> 216 us; 256^3 learned V-cycle 661 -> 651 us.)
 //   warp 0      TMA producer: per brick one (two with the pair) box;
 //   warp 1      TMEM owner and MMA issuer, two accumulators of 4 x 16 columns;
 //   warps 2-5   epilogue.
@@ -650,9 +707,8 @@ __global__ void __launch_bounds__(k3Threads, 1)
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
-    const int tx = (g.nx + kOX - 1) / kOX, ty = (g.ny + kTY - 1) / kTY, tz = (g.nz + kTZ - 1) / kTZ;
-    const long per_sample = (long)tx * ty * tz;
-    const long ntiles = per_sample * g.nb;
+    BrickWalk walk(g, kOX, kTY, kTZ, blockIdx.x, gridDim.x);
+    const long ntiles = walk.count(g.nb);
 
     // weight tile (dy, dz): column dx + 1 takes that tap, the others are zero
     for(int i = tid; i < k3Tiles * k3PlaneCols * kNetCh; i += k3Threads)
@@ -696,12 +752,12 @@ __global__ void __launch_bounds__(k3Threads, 1)
     {
         // ---- TMA producer
         long issued = 0;
-        for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++issued)
+        for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, walk.next(), ++issued)
         {
             const int st = (int)(issued % k3Stages);
             const uint32_t ph = (uint32_t)((issued / k3Stages) & 1);
             if(!role_wait(&empty[st], ph ^ 1u, abort_flag, status, 3)) break;
-            const Brick bk = brick_of(g, tile, tx, ty, per_sample);
+            const Brick bk = walk.at(kOX, kTY, kTZ);
             mbar_expect_tx(&full[st], kBoxTx);
             unsigned char* dst = sA + st * k3StageBytes;
             tma_load_5d(dst, &in_map, 0, bk.x0 - 1, bk.y0 - 1, bk.z0 - 1, bk.b, &full[st]);
@@ -715,9 +771,9 @@ __global__ void __launch_bounds__(k3Threads, 1)
                 mbar_wait(&full[k % k3Stages], (uint32_t)((k / k3Stages) & 1));
         }
     }
-    else if(warp == 1 && lane == 0)
+    else if(warp == 1)
     {
-        // ---- MMA issuer
+        // ---- MMA issuer: the whole warp walks the loop, one elected lane issues
         const uint64_t bd = umma_desc(smem_u32(sW), 128, 256);
         long i = 0;
         for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++i)
@@ -726,44 +782,49 @@ __global__ void __launch_bounds__(k3Threads, 1)
             const uint32_t ph = (uint32_t)((i / k3Stages) & 1);
             const int acc = (int)(i & 1);
             const uint32_t aph = (uint32_t)((i >> 1) & 1);
-            if(!role_wait(&tempty[acc], aph ^ 1u, abort_flag, status, 4)) break;
-            if(!role_wait(&full[st], ph, abort_flag, status, 5)) break;
+            const bool ready = role_wait(&tempty[acc], aph ^ 1u, abort_flag, status, 4) &&
+                               role_wait(&full[st], ph, abort_flag, status, 5);
+            if(!__all_sync(0xffffffffu, ready)) break;
             tc_fence_after();
             const uint64_t a0 = umma_desc_sw32(smem_u32(sA + st * k3StageBytes));
             const uint32_t d0 = tmem + (uint32_t)(acc * k3AccCols);
             // as in k_conv16: plane q feeds output planes mt in [lo, hi] with dz
             // tile mt - q + 2, and first writes plane q by an MMA of its own
-#pragma unroll
-            for(int q = 0; q < kTZ + 2; ++q)
+            if(elect_one())
             {
-                const int lo = q - 2 < 0 ? 0 : q - 2;
-                const int hi = q < kTZ - 1 ? q : kTZ - 1;
 #pragma unroll
-                for(int dyi = 0; dyi < 3; ++dyi)
+                for(int q = 0; q < kTZ + 2; ++q)
                 {
-                    const uint64_t ad = a0 + (uint64_t)(((q * kHY + dyi) * kTX * kRowBytes) >> 4);
-                    auto mma = [&](int m0, int m1, uint32_t accumulate) {
-                        const uint32_t idesc = umma_idesc_bf16(128, (m1 - m0 + 1) * k3PlaneCols, false, false);
-                        const uint64_t bs = bd + (uint64_t)(((dyi * 3 + m0 - q + 2) * k3Tile) >> 4);
-                        const uint32_t d = d0 + (uint32_t)(m0 * k3PlaneCols);
-                        mma_bf16(d, ad, bs, idesc, accumulate);
-                        if(kPair)
-                            mma_bf16(d, ad + (uint64_t)(k3BoxBytes >> 4), bs + (uint64_t)((k3Tiles * k3Tile) >> 4),
-                                     idesc, 1u);
-                    };
-                    if(q <= kTZ - 1 && dyi == 0)
+                    const int lo = q - 2 < 0 ? 0 : q - 2;
+                    const int hi = q < kTZ - 1 ? q : kTZ - 1;
+#pragma unroll
+                    for(int dyi = 0; dyi < 3; ++dyi)
                     {
-                        if(hi > lo) mma(lo, hi - 1, 1u);
-                        mma(hi, hi, 0u);
-                    }
-                    else
-                    {
-                        mma(lo, hi, 1u);
+                        const uint64_t ad = a0 + (uint64_t)(((q * kHY + dyi) * kTX * kRowBytes) >> 4);
+                        auto mma = [&](int m0, int m1, uint32_t accumulate) {
+                            const uint32_t idesc = umma_idesc_bf16(128, (m1 - m0 + 1) * k3PlaneCols, false, false);
+                            const uint64_t bs = bd + (uint64_t)(((dyi * 3 + m0 - q + 2) * k3Tile) >> 4);
+                            const uint32_t d = d0 + (uint32_t)(m0 * k3PlaneCols);
+                            mma_bf16(d, ad, bs, idesc, accumulate);
+                            if(kPair)
+                                mma_bf16(d, ad + (uint64_t)(k3BoxBytes >> 4), bs + (uint64_t)((k3Tiles * k3Tile) >> 4),
+                                         idesc, 1u);
+                        };
+                        if(q <= kTZ - 1 && dyi == 0)
+                        {
+                            if(hi > lo) mma(lo, hi - 1, 1u);
+                            mma(hi, hi, 0u);
+                        }
+                        else
+                        {
+                            mma(lo, hi, 1u);
+                        }
                     }
                 }
+                mma_commit(&empty[st]);   // stage free once these MMAs have read it
+                mma_commit(&tfull[acc]);  // accumulator ready for the epilogue
             }
-            mma_commit(&empty[st]);   // stage free once these MMAs have read it
-            mma_commit(&tfull[acc]);  // accumulator ready for the epilogue
+            __syncwarp();
         }
         if(*abort_flag && i > 0)
         {
@@ -778,7 +839,7 @@ __global__ void __launch_bounds__(k3Threads, 1)
         const int qd = warp & 3;
         const int m = qd * 32 + lane;
         long i = 0;
-        for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++i)
+        for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, walk.next(), ++i)
         {
             const int acc = (int)(i & 1);
             const uint32_t aph = (uint32_t)((i >> 1) & 1);
@@ -789,7 +850,7 @@ __global__ void __launch_bounds__(k3Threads, 1)
             tmem_ld4x4(tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(acc * k3AccCols), k3PlaneCols, v);
             tc_fence_before();
             mbar_arrive(&tempty[acc]);  // the accumulator may take the next brick
-            const Brick bk = brick_of(g, tile, tx, ty, per_sample);
+            const Brick bk = walk.at(kOX, kTY, kTZ);
             // row m is staged point (xi, yi) of a plane; xi = 0 and kTX - 1 are the halo columns
             const int xi = m % kTX;
             const int x = bk.x0 - 1 + xi, y = bk.y0 + m / kTX;
@@ -840,7 +901,8 @@ __global__ void __launch_bounds__(k3Threads, 1)
 // MMAs from one elected lane (72 a unit, 40 cycles each; issued by a loader thread
 // between two block barriers they took 53, and loads and MMAs met at each unit).
 // A training batch of 64 samples of 16^3 (three weight gradients, two
-// convolutions): im2col 1572 us, bricks 361, with the warps' split 299.
+// convolutions): im2col 1572 us, bricks 361, with the warps' split 299
+// (289 with the forward passes' carried coordinates).
 constexpr int kWgX = 16, kWgLines = 3, kWgZ = 8;                  // gradient points of a unit
 constexpr int kWgXA = kWgX + 2, kWgLinesA = kWgLines + 2, kWgZA = kWgZ + 2;  // input points, with the halo
 constexpr int kWgRowA = kWgXA * 16, kWgRowB = kWgX * 16;          // bytes of one line of one half
@@ -906,14 +968,11 @@ __global__ void __launch_bounds__(kWgThreads + 32, 1)
     {
         // ---- loaders: 16-byte items of unit u (plane, line, x, half), zero outside the sample
         uint4 va[kWgLoadsA], vb[kWgLoadsB];
-        auto load = [&](long u) {
-            const int bx = (int)(u % U.tx);
-            const long q1 = u / U.tx;
-            const int by = (int)(q1 % U.ty);
-            const long q2 = q1 / U.ty;
-            const int bz = (int)(q2 % U.tz);
-            const long b = q2 / U.tz;
-            const int x0 = bx * kWgX, y0 = by * kWgLines, z0 = bz * kWgZ;
+        BrickWalk walk(g, kWgX, kWgLines, kWgZ, blockIdx.x, gridDim.x);
+        auto load = [&] {
+            const Brick bk = walk.at(kWgX, kWgLines, kWgZ);
+            const long b = bk.b;
+            const int x0 = bk.x0, y0 = bk.y0, z0 = bk.z0;
             auto fetch = [&](const __nv_bfloat16* src, int z, int y, int xx, int half) {
                 if((unsigned)z >= (unsigned)g.nz || (unsigned)y >= (unsigned)g.ny || (unsigned)xx >= (unsigned)g.nx)
                     return make_uint4(0, 0, 0, 0);
@@ -936,7 +995,7 @@ __global__ void __launch_bounds__(kWgThreads + 32, 1)
                                       : make_uint4(0, 0, 0, 0);
             }
         };
-        load(blockIdx.x);
+        load();
         int k = 0;
         for(long u = blockIdx.x; u < U.count; u += gridDim.x, ++k)
         {
@@ -960,7 +1019,8 @@ __global__ void __launch_bounds__(kWgThreads + 32, 1)
             }
             fence_async_smem();
             mbar_arrive(&full[st]);
-            if(u + gridDim.x < U.count) load(u + gridDim.x);
+            walk.next();
+            if(u + gridDim.x < U.count) load();
         }
     }
     else
@@ -1320,23 +1380,18 @@ __global__ void __launch_bounds__(k1Threads) k_layer1_tc(ConvGrid g, const Tin* 
     pdl_wait();  // from here on the previous kernel's output is read
 
     const long n = g.points();
-    const int tx = (g.nx + k1X - 1) / k1X, ty = (g.ny + k1Y - 1) / k1Y, tz = (g.nz + k1Z - 1) / k1Z;
-    const long per_sample = (long)tx * ty * tz;
-    const long ntiles = per_sample * g.nb;
+    BrickWalk walk(g, k1X, k1Y, k1Z, blockIdx.x, gridDim.x);
+    const long ntiles = walk.count(g.nb);
     constexpr uint32_t idesc = umma_idesc_bf16(128, kNetCh, false, false);
     const uint64_t bd = umma_desc(smem_u32(sW), 128, 512);
     const int mx = tid % k1X, my = tid / k1X;
     uint32_t phase = 0;
     bool failed = false;
-    for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
+    for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, walk.next())
     {
-        const int b = (int)(tile / per_sample);
-        long t2 = tile - (long)b * per_sample;
-        const int bz = (int)(t2 / ((long)tx * ty));
-        t2 -= (long)bz * tx * ty;
-        const int by = (int)(t2 / tx), bx = (int)(t2 - (long)by * tx);
-        const int x0 = bx * k1X, y0 = by * k1Y, z0 = bz * k1Z;
-        const long base = (long)b * g.nz * g.ny * g.nx;
+        const Brick bk = walk.at(k1X, k1Y, k1Z);
+        const int x0 = bk.x0, y0 = bk.y0, z0 = bk.z0;
+        const long base = (long)bk.b * g.nz * g.ny * g.nx;
         for(int e = tid; e < k1Halo; e += k1Threads)
         {
             const int hx = e % k1HX, hy = (e / k1HX) % k1HY, hz = e / (k1HX * k1HY);
