@@ -239,12 +239,28 @@ __device__ __forceinline__ int perm_row(const PermMap& pm, int z, int y, int x)
     return pm.offsets[v] + ((z >> 1) * pm.by[v] + (y >> 1)) * pm.bx[v] + (x >> 1);
 }
 
+__device__ __forceinline__ uint32_t pack_bf16x2(float a, float b)
+{
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
 __device__ __forceinline__ uint4 pack_bf16x8(const float* v)
 {
     __align__(16) __nv_bfloat162 h[4];
 #pragma unroll
     for(int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
     return *reinterpret_cast<uint4*>(h);
+}
+
+// The 32 bytes of one point's 16 BF16 channels in one access (256-bit, sm_100):
+// two 16-byte ones each touch half of every sector of the warp's points.  p is
+// 32-byte aligned.
+__device__ __forceinline__ void store_point(void* p, uint4 a, uint4 b)
+{
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
+                 "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
 }
 
 // K-major no-swizzle offset (bytes) of row r, 8-element K chunk c, for
@@ -552,6 +568,7 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
         constexpr int kPlanes = kTZ / 2;
         static_assert(kPlanes == 2 && kPlaneCols == 48, "two planes a warp");
         const int mt0 = (warp - 2) / 4 * kPlanes;  // this warp's output planes of a brick
+        const bool wide = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
         long i = 0;
         for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, walk.next(), ++i)
         {
@@ -614,8 +631,12 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
                         for(int c = 0; c < 16; ++c) v[c] = __bfloat162float(h[c]) > 0.f ? v[c] : 0.f;
                     }
                     uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(out) + p * kNetCh);
-                    dst[0] = pack_bf16x8(v);
-                    dst[1] = pack_bf16x8(v + 8);
+                    if(wide) store_point(dst, pack_bf16x8(v), pack_bf16x8(v + 8));
+                    else
+                    {
+                        dst[0] = pack_bf16x8(v);
+                        dst[1] = pack_bf16x8(v + 8);
+                    }
                 }
                 else if constexpr(kOut == kOutF32)
                 {
@@ -1320,48 +1341,55 @@ __device__ __forceinline__ float in_value(const float* v, long q) { return __bfl
 
 // ------------------------------------------------------------ layer 1 (1 -> 16)
 //
-// One input channel: the 27 taps are the K dimension.  Per brick of
-// 16 x 8 x 4 points the CTA stages the halo'd scalar field (18 x 10 x 6,
-// BF16-rounded, zero outside the grid), each thread writes the im2col row of
-// its point in every z plane (27 neighbours, 5 zeros: K = 32), and two MMAs
-// per plane (M = 128 points, N = 16 channels, K = 16 each) give the 16
-// pre-activations in TMEM; the epilogue writes relu(z) and, for the odd pair,
-// relu(-z) as BF16.  Several CTAs per SM overlap one CTA's MMA round trip with
-// the others' staging.
+// One input channel: the 27 taps are the K dimension, of two MMAs per plane of a
+// 16 x 8 x 4 brick (M = 128 points, N = 16 channels, K = 16 each, 5 zero taps).
+// What bounds it: it has 64 B a point of the odd pair to write; gathering every
+// point's 27 neighbours from a staged field and rounding each again cost 57 us on
+// a 128^3 sample.  Here A is MN-major: eight points along x are the 16 bytes of
+// one tap.  A thread reads ten points of one line of the halo'd brick, rounds
+// them once, and the three shifted runs of eight (dx = -1, 0, +1) are stored for
+// each of the up to nine (dz, dy) the line serves: 27 16-byte stores for 240
+// values.  Tap runs of an 8-point group are contiguous (K core matrices 128 B
+// apart), groups 528 B apart, which spreads a store over all banks.  The
+// epilogue writes relu(z) and, for the odd pair, relu(-z) as BF16, a point's 32
+// bytes at a time (in two halves the stores were the bound: the new gather alone
+// gained 1 us, with whole points 45).  The next brick's points are on their way
+// meanwhile, and several CTAs per SM overlap.
 constexpr int k1X = 16, k1Y = 8, k1Z = 4;
-constexpr int k1HX = k1X + 2, k1HY = k1Y + 2, k1HZ = k1Z + 2;
-constexpr int k1Halo = k1HX * k1HY * k1HZ;  // 1080 staged scalars
-constexpr int k1Threads = 128;              // one thread per point of a plane
-constexpr int k1K = 32;                     // 27 taps + 5 zeros
-constexpr int k1PlaneBytes = 128 * k1K * 2; // 8 KB of im2col rows per plane
-constexpr int k1Cols = k1Z * kNetCh;        // TMEM columns per brick
-constexpr int k1WBytes = kNetCh * k1K * 2;  // B: 16 channel rows x 32 taps
-constexpr int k1Smem = k1Z * k1PlaneBytes + k1WBytes + k1Halo * 4 + 64 + 1024;
-constexpr int k1CtasPerSm = 4;
+constexpr int k1Threads = 128;               // one thread per point of a plane
+constexpr int k1Lines = 2 * (k1Y + 2) * (k1Z + 2);  // (plane, line, 8-point half) of the halo'd brick: a thread each
+constexpr int k1K = 32;                      // 27 taps + 5 zeros
+constexpr int k1Group = k1K * 16 + 16;       // bytes of an 8-point group
+constexpr int k1PlaneBytes = 16 * k1Group;
+constexpr int k1Cols = k1Z * kNetCh;         // TMEM columns per brick
+constexpr int k1WBytes = kNetCh * k1K * 2;   // B: 16 channel rows x 32 taps
+constexpr int k1Smem = k1Z * k1PlaneBytes + k1WBytes + 128;
+constexpr int k1CtasPerSm = 6;
 
-static_assert(k1X * k1Y == k1Threads, "one plane of the brick is one 128-row M tile");
+static_assert(k1X * k1Y == k1Threads && k1X == 16, "one plane of the brick is one 128-row M tile");
+static_assert(k1Lines <= k1Threads, "a thread per staged line");
 static_assert(k1Cols * k1CtasPerSm <= 512, "TMEM columns of the co-resident CTAs");
+static_assert(k1CtasPerSm * (k1Smem + 1024) <= 227 * 1024, "shared memory of the co-resident CTAs");
 
-// K-major no-swizzle offset of row r, 8-element K chunk c8 of a 32-wide K
-// operand: chunks 128 B apart (LBO), 8-row groups 512 B apart (SBO).
+// K-major no-swizzle offset of row r, 8-element K chunk c8 of the weights' 32-wide
+// K: chunks 128 B apart (LBO), 8-row groups 512 B apart (SBO).
 __host__ __device__ constexpr uint32_t k1_off(int r, int c8)
 {
     return (uint32_t)((r >> 3) * 512 + c8 * 128 + (r & 7) * 16);
 }
 
 template <typename Tin, bool kPair>
-__global__ void __launch_bounds__(k1Threads) k_layer1_tc(ConvGrid g, const Tin* __restrict__ in,
-                                                         const float* __restrict__ w1,
-                                                         __nv_bfloat16* __restrict__ a1, int* status)
+__global__ void __launch_bounds__(k1Threads, k1CtasPerSm)
+    k_layer1_tc(ConvGrid g, const Tin* __restrict__ in, const float* __restrict__ w1, __nv_bfloat16* __restrict__ a1,
+                int* status)
 {
     extern __shared__ unsigned char smem_raw[];
     pdl_launch_dependents();  // the next kernel may start its prologue
-    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    unsigned char* sA = smem;                           // k1Z im2col planes
-    unsigned char* sW = sA + k1Z * k1PlaneBytes;        // weights
-    float* sS = (float*)(sW + k1WBytes);                // staged scalars
-    uint64_t* mbar = (uint64_t*)(sS + k1Halo);
-    uint32_t* tholder = (uint32_t*)(mbar + 1);
+    unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
+    unsigned char* sA = smem;                     // k1Z planes of tap runs
+    unsigned char* sW = sA + k1Z * k1PlaneBytes;  // weights
+    __shared__ uint64_t mbar;
+    __shared__ uint32_t tholder;
 
     const int tid = threadIdx.x, warp = tid >> 5;
     for(int i = tid; i < kNetCh * k1K; i += k1Threads)
@@ -1370,111 +1398,121 @@ __global__ void __launch_bounds__(k1Threads) k_layer1_tc(ConvGrid g, const Tin* 
         const float w = t < 27 ? w1[t * kNetCh * kNetCh + co] : 0.f;  // w1[t][0][co]
         *reinterpret_cast<__nv_bfloat16*>(sW + k1_off(co, t >> 3) + (t & 7) * 2) = __float2bfloat16_rn(w);
     }
-    if(tid == 0) mbar_init(mbar, 1);
-    if(warp == 0) tmem_alloc(tholder, k1Cols);
+    // the zero taps stay
+    for(int i = tid; i < k1Z * 16 * (k1K - 27); i += k1Threads)
+        *reinterpret_cast<uint4*>(sA + i / (k1K - 27) * k1Group + (27 + i % (k1K - 27)) * 16) = make_uint4(0, 0, 0, 0);
+    if(tid == 0) mbar_init(&mbar, 1);
+    if(warp == 0) tmem_alloc(&tholder, k1Cols);
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = *tholder;
+    const uint32_t tmem = tholder;
     pdl_wait();  // from here on the previous kernel's output is read
 
     const long n = g.points();
     BrickWalk walk(g, k1X, k1Y, k1Z, blockIdx.x, gridDim.x);
     const long ntiles = walk.count(g.nb);
-    constexpr uint32_t idesc = umma_idesc_bf16(128, kNetCh, false, false);
-    const uint64_t bd = umma_desc(smem_u32(sW), 128, 512);
-    const int mx = tid % k1X, my = tid / k1X;
-    uint32_t phase = 0;
-    bool failed = false;
-    for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, walk.next())
-    {
+    constexpr uint32_t idesc = umma_idesc_bf16(128, kNetCh, true, false);
+    const uint64_t ad = umma_desc(smem_u32(sA), 128, k1Group), bd = umma_desc(smem_u32(sW), 128, 512);
+    const int mx = tid % k1X, my = tid / k1X;                           // this thread's point of each plane
+    const int half = tid & 1, hy = (tid >> 1) % (k1Y + 2), hz = (tid >> 1) / (k1Y + 2);  // and staged line
+
+    // points x0 + 8 half - 1 .. + 8 of the line, zero outside the sample
+    float v[10];
+    auto load = [&] {
         const Brick bk = walk.at(k1X, k1Y, k1Z);
-        const int x0 = bk.x0, y0 = bk.y0, z0 = bk.z0;
-        const long base = (long)bk.b * g.nz * g.ny * g.nx;
-        for(int e = tid; e < k1Halo; e += k1Threads)
+        const int x = bk.x0 + 8 * half - 1, y = bk.y0 + hy - 1, z = bk.z0 + hz - 1;
+        const bool line = tid < k1Lines && (unsigned)y < (unsigned)g.ny && (unsigned)z < (unsigned)g.nz;
+        const long at = (((long)bk.b * g.nz + z) * g.ny + y) * g.nx + x;
+#pragma unroll
+        for(int i = 0; i < 10; ++i)
+            v[i] = line && (unsigned)(x + i) < (unsigned)g.nx ? in_value(in, at + i) : 0.f;
+    };
+    load();
+    uint32_t phase = 0;
+    bool ok = true;
+    for(long tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
+    {
+        if(tid < k1Lines)
         {
-            const int hx = e % k1HX, hy = (e / k1HX) % k1HY, hz = e / (k1HX * k1HY);
-            const int x = x0 + hx - 1, y = y0 + hy - 1, z = z0 + hz - 1;
-            float v = 0.f;
-            if(x >= 0 && x < g.nx && y >= 0 && y < g.ny && z >= 0 && z < g.nz)
-                v = in_value(in, base + ((long)z * g.ny + y) * g.nx + x);
-            sS[e] = v;
+            uint32_t p[5], q[4];  // pairs (0,1) (2,3) .. and (1,2) (3,4) ..
+#pragma unroll
+            for(int i = 0; i < 5; ++i) p[i] = pack_bf16x2(v[2 * i], v[2 * i + 1]);
+#pragma unroll
+            for(int i = 0; i < 4; ++i) q[i] = pack_bf16x2(v[2 * i + 1], v[2 * i + 2]);
+#pragma unroll
+            for(int dz = 0; dz < 3; ++dz)
+#pragma unroll
+                for(int dy = 0; dy < 3; ++dy)
+                {
+                    // the output plane and line whose tap (dz - 1, dy - 1) this line is
+                    const int oz = hz - dz, oy = hy - dy;
+                    if((unsigned)oz >= (unsigned)k1Z || (unsigned)oy >= (unsigned)k1Y) continue;
+                    uint4* run = reinterpret_cast<uint4*>(sA + oz * k1PlaneBytes + (2 * oy + half) * k1Group) +
+                                 dz * 9 + dy * 3;
+                    run[0] = make_uint4(p[0], p[1], p[2], p[3]);
+                    run[1] = make_uint4(q[0], q[1], q[2], q[3]);
+                    run[2] = make_uint4(p[1], p[2], p[3], p[4]);
+                }
         }
-        __syncthreads();
-#pragma unroll 1
-        for(int q = 0; q < k1Z; ++q)
-        {
-            __align__(16) __nv_bfloat16 h[k1K];
-#pragma unroll
-            for(int t = 0; t < 27; ++t)
-            {
-                const int dz = t / 9 - 1, dy = (t / 3) % 3 - 1, dx = t % 3 - 1;
-                h[t] = __float2bfloat16_rn(sS[((q + 1 + dz) * k1HY + (my + 1 + dy)) * k1HX + (mx + 1 + dx)]);
-            }
-#pragma unroll
-            for(int t = 27; t < k1K; ++t) h[t] = __float2bfloat16_rn(0.f);
-            unsigned char* row = sA + q * k1PlaneBytes;
-#pragma unroll
-            for(int c8 = 0; c8 < k1K / 8; ++c8)
-                *reinterpret_cast<uint4*>(row + k1_off(tid, c8)) = *reinterpret_cast<const uint4*>(h + 8 * c8);
-        }
-        fence_async_smem();  // the im2col rows are read by the tensor cores
+        fence_async_smem();  // the runs are read by the tensor cores
         tc_fence_before();
-        __syncthreads();
+        if(__syncthreads_or(!ok)) break;
         tc_fence_after();
-        if(tid == 0)
+        if(warp == 0 && elect_one())
         {
 #pragma unroll
-            for(int q = 0; q < k1Z; ++q)
+            for(int z = 0; z < k1Z; ++z)
 #pragma unroll
                 for(int kh = 0; kh < 2; ++kh)
-                    mma_bf16(tmem + q * kNetCh, umma_desc(smem_u32(sA + q * k1PlaneBytes + kh * 256), 128, 512),
+                    mma_bf16(tmem + z * kNetCh, ad + (uint64_t)((z * k1PlaneBytes + kh * 256) >> 4),
                              bd + (uint64_t)((kh * 256) >> 4), idesc, (uint32_t)kh);
-            mma_commit(mbar);
+            mma_commit(&mbar);
         }
-        const bool ok = mbar_wait(mbar, phase);
+        __syncwarp();
+        const Brick bk = walk.at(k1X, k1Y, k1Z);
+        walk.next();
+        if(tile + gridDim.x < ntiles) load();
+        ok = __all_sync(0xffffffffu, mbar_wait(&mbar, phase));
+        if(!ok) continue;  // the block leaves together
         phase ^= 1u;
-        if(__syncthreads_or(!ok))
-        {
-            if(tid == 0) atomicExch(status, 7);
-            failed = true;
-            break;
-        }
         tc_fence_after();
+        const int x = bk.x0 + mx, y = bk.y0 + my;
+        const long row = (((long)bk.b * g.nz + bk.z0) * g.ny + y) * g.nx + x;
 #pragma unroll 1
-        for(int q = 0; q < k1Z; ++q)
+        for(int z = 0; z < k1Z; ++z)
         {
-            float v[16];
-            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(q * kNetCh), v);
-            const int x = x0 + mx, y = y0 + my, z = z0 + q;
-            if(x >= g.nx || y >= g.ny || z >= g.nz) continue;
-            const long p = base + ((long)z * g.ny + y) * g.nx + x;
-            float pos[16];
-#pragma unroll
-            for(int c = 0; c < 16; ++c) pos[c] = fmaxf(v[c], 0.f);
-            uint4* dst = reinterpret_cast<uint4*>(a1 + p * kNetCh);
-            dst[0] = pack_bf16x8(pos);
-            dst[1] = pack_bf16x8(pos + 8);
-            if(kPair)
+            float s[16];
+            tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(z * kNetCh), s);
+            if(x < g.nx && y < g.ny && bk.z0 + z < g.nz)
             {
+                const long pt = row + (long)z * g.ny * g.nx;
+                float pos[16];
 #pragma unroll
-                for(int c = 0; c < 16; ++c) pos[c] = fmaxf(-v[c], 0.f);
-                uint4* d2 = reinterpret_cast<uint4*>(a1 + (p + n) * kNetCh);
-                d2[0] = pack_bf16x8(pos);
-                d2[1] = pack_bf16x8(pos + 8);
+                for(int c = 0; c < 16; ++c) pos[c] = fmaxf(s[c], 0.f);
+                store_point(a1 + pt * kNetCh, pack_bf16x8(pos), pack_bf16x8(pos + 8));
+                if(kPair)
+                {
+#pragma unroll
+                    for(int c = 0; c < 16; ++c) pos[c] = fmaxf(-s[c], 0.f);
+                    store_point(a1 + (pt + n) * kNetCh, pack_bf16x8(pos), pack_bf16x8(pos + 8));
+                }
             }
+            __syncwarp();
         }
-        tc_fence_before();
-        __syncthreads();  // TMEM, im2col planes and staged scalars free for the next brick
     }
-    if(failed) mbar_wait(mbar, phase ^ 1u);  // the MMAs in flight finish before TMEM is released
     tc_fence_before();
-    __syncthreads();
+    const bool failed = __syncthreads_or(!ok);
+    if(failed)
+    {
+        if(tid == 0) atomicExch(status, 7);
+        if(!ok) mbar_wait(&mbar, phase);  // the MMAs in flight finish before TMEM is released
+        __syncthreads();
+    }
     tc_fence_after();
     if(warp == 0) tmem_free(tmem, k1Cols);
 }
-
 
 // 1 / (e.e) (kind 0) or 1 / (e.Ae) (kind 1) per sample: one block per sample.
 __global__ void k_sample_norm(ConvGrid g, const float* __restrict__ e, int kind, float* __restrict__ out)
