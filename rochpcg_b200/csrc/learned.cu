@@ -923,7 +923,8 @@ __global__ void __launch_bounds__(k3Threads, 1)
 // between two block barriers they took 53, and loads and MMAs met at each unit).
 // A training batch of 64 samples of 16^3 (three weight gradients, two
 // convolutions): im2col 1572 us, bricks 361, with the warps' split 299
-// (289 with the forward passes' carried coordinates).
+// (289 with the forward passes' carried coordinates, 266 with the one-channel
+// forms of layers 1 and 3 in the forward pass and of layer 3's gradient).
 constexpr int kWgX = 16, kWgLines = 3, kWgZ = 8;                  // gradient points of a unit
 constexpr int kWgXA = kWgX + 2, kWgLinesA = kWgLines + 2, kWgZA = kWgZ + 2;  // input points, with the halo
 constexpr int kWgRowA = kWgXA * 16, kWgRowB = kWgX * 16;          // bytes of one line of one half
@@ -1151,9 +1152,7 @@ __global__ void k_prepare_weights(const float* __restrict__ w, __nv_bfloat16* __
 __device__ __forceinline__ void store_embed(__nv_bfloat16* a, long p, float r0)
 {
     const float v[8] = {r0, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    uint4* dst = reinterpret_cast<uint4*>(a + p * kNetCh);
-    dst[0] = pack_bf16x8(v);
-    dst[1] = make_uint4(0, 0, 0, 0);
+    store_point(a + p * kNetCh, pack_bf16x8(v), make_uint4(0, 0, 0, 0));
 }
 
 // Channel 0 = r (x == nullptr) or the residual r - A x of the 27-point
@@ -1378,10 +1377,14 @@ __host__ __device__ constexpr uint32_t k1_off(int r, int c8)
     return (uint32_t)((r >> 3) * 512 + c8 * 128 + (r & 7) * 16);
 }
 
-template <typename Tin, bool kPair>
+// kMask: the gradient of layer 3 instead.  in is dL/dy (one value a point, the
+// second branch's being its negative), w1 are layer 3's weights, used transposed,
+// and the result is kept where act > 0.  (As a 16 -> 16 convolution of dL/dy with
+// 15 zero channels: 30 us on 2 x 64 samples of 16^3, here 18.)
+template <typename Tin, bool kPair, bool kMask>
 __global__ void __launch_bounds__(k1Threads, k1CtasPerSm)
     k_layer1_tc(ConvGrid g, const Tin* __restrict__ in, const float* __restrict__ w1, __nv_bfloat16* __restrict__ a1,
-                int* status)
+                const __nv_bfloat16* __restrict__ act, int* status)
 {
     extern __shared__ unsigned char smem_raw[];
     pdl_launch_dependents();  // the next kernel may start its prologue
@@ -1395,7 +1398,9 @@ __global__ void __launch_bounds__(k1Threads, k1CtasPerSm)
     for(int i = tid; i < kNetCh * k1K; i += k1Threads)
     {
         const int co = i / k1K, t = i % k1K;
-        const float w = t < 27 ? w1[t * kNetCh * kNetCh + co] : 0.f;  // w1[t][0][co]
+        // w1[t][0][co], or w3[26 - t][co][0]
+        const int at = kMask ? (26 - t) * kNetCh * kNetCh + co * kNetCh : t * kNetCh * kNetCh + co;
+        const float w = t < 27 ? w1[at] : 0.f;
         *reinterpret_cast<__nv_bfloat16*>(sW + k1_off(co, t >> 3) + (t & 7) * 2) = __float2bfloat16_rn(w);
     }
     // the zero taps stay
@@ -1483,20 +1488,38 @@ __global__ void __launch_bounds__(k1Threads, k1CtasPerSm)
 #pragma unroll 1
         for(int z = 0; z < k1Z; ++z)
         {
+            const bool inside = x < g.nx && y < g.ny && bk.z0 + z < g.nz;
+            const long pt = row + (long)z * g.ny * g.nx;
+            uint4 m[kMask ? 4 : 1];
+            if constexpr(kMask)
+            {
+#pragma unroll
+                for(int i = 0; i < (kPair ? 4 : 2); ++i)
+                    m[i] = inside ? __ldg(reinterpret_cast<const uint4*>(act + (pt + (i >> 1) * n) * kNetCh) + (i & 1))
+                                  : make_uint4(0, 0, 0, 0);
+            }
             float s[16];
             tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(z * kNetCh), s);
-            if(x < g.nx && y < g.ny && bk.z0 + z < g.nz)
+            if(inside)
             {
-                const long pt = row + (long)z * g.ny * g.nx;
-                float pos[16];
 #pragma unroll
-                for(int c = 0; c < 16; ++c) pos[c] = fmaxf(s[c], 0.f);
-                store_point(a1 + pt * kNetCh, pack_bf16x8(pos), pack_bf16x8(pos + 8));
-                if(kPair)
+                for(int br = 0; br < (kPair ? 2 : 1); ++br)
                 {
+                    float o[16];
+                    __align__(16) __nv_bfloat16 h[kMask ? 16 : 8];
+                    if constexpr(kMask)
+                    {
+                        *reinterpret_cast<uint4*>(h) = m[2 * br];
+                        *reinterpret_cast<uint4*>(h + 8) = m[2 * br + 1];
+                    }
 #pragma unroll
-                    for(int c = 0; c < 16; ++c) pos[c] = fmaxf(-s[c], 0.f);
-                    store_point(a1 + (pt + n) * kNetCh, pack_bf16x8(pos), pack_bf16x8(pos + 8));
+                    for(int c = 0; c < 16; ++c)
+                    {
+                        const float v = br ? -s[c] : s[c];
+                        if constexpr(kMask) o[c] = __bfloat162float(h[c]) > 0.f ? v : 0.f;
+                        else o[c] = fmaxf(v, 0.f);
+                    }
+                    store_point(a1 + (pt + br * n) * kNetCh, pack_bf16x8(o), pack_bf16x8(o + 8));
                 }
             }
             __syncwarp();
@@ -1531,23 +1554,21 @@ __global__ void k_sample_norm(ConvGrid g, const float* __restrict__ e, int kind,
 }
 
 // d = y - e, y the network output (odd: (y[p] - y[p + n]) / 2).
-__global__ void k_loss_diff(long n, const float* __restrict__ y, const float* __restrict__ e, int odd,
-                            float* __restrict__ d)
+__global__ void k_loss_diff(long n, const float* __restrict__ y, const float* __restrict__ e, float* __restrict__ d)
 {
     const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if(p >= n) return;
-    const float yv = odd ? 0.5f * (y[p] - y[p + n]) : y[p];
-    d[p] = yv - e[p];
+    if(p < n) d[p] = y[p] - e[p];
 }
 
 constexpr int kLossBlocks = 1184;
 
 // Loss terms d.Md * w (M = I for kind 0, the stencil A for kind 1, i.e. the
 // error's energy norm) and the output gradient 2 M d w as BF16 channel 0 of
-// G (odd: +/- half of it for the two branches).
+// G (odd: +/- half of it for the two branches), and of the first branch in gy.
 __global__ void __launch_bounds__(256) k_loss_grad(ConvGrid g, const float* __restrict__ d,
                                                    const float* __restrict__ wnorm, float scale, int kind, int odd,
-                                                   __nv_bfloat16* __restrict__ G, float* __restrict__ loss_partial)
+                                                   __nv_bfloat16* __restrict__ G, float* __restrict__ gy,
+                                                   float* __restrict__ loss_partial)
 {
     __shared__ float red[32];
     const long per = (long)g.nz * g.ny * g.nx;
@@ -1558,16 +1579,10 @@ __global__ void __launch_bounds__(256) k_loss_grad(ConvGrid g, const float* __re
         const float w = wnorm[p / per] * scale;
         const float md = kind ? stencil_at(g, d, p) : d[p];
         acc += d[p] * md * w;
-        const float gv = 2.f * md * w;
-        if(odd)
-        {
-            store_embed(G, p, 0.5f * gv);
-            store_embed(G, p + n, -0.5f * gv);
-        }
-        else
-        {
-            store_embed(G, p, gv);
-        }
+        const float gv = (odd ? 1.f : 2.f) * md * w;
+        gy[p] = gv;
+        store_embed(G, p, gv);
+        if(odd) store_embed(G, p + n, -gv);
     }
     acc = block_sum(acc, red);
     if(threadIdx.x == 0) loss_partial[blockIdx.x] = acc;
@@ -1815,33 +1830,40 @@ int launch_embed_scalar_level(const PermMap& pm, int nz, int ny, int nx, const f
 }
 
 
-template <typename Tin, bool kPair>
-static int layer1_launch(const ConvGrid& g, const Tin* in, const float* w1, __nv_bfloat16* a1, int* status,
+template <typename Tin, bool kPair, bool kMask = false>
+static int layer1_launch(const ConvGrid& g, const Tin* in, const float* w1, void* a1, const void* act, int* status,
                          cudaStream_t s)
 {
     static bool attr = false;
     if(!attr)
     {
-        HB_CUDA(cudaFuncSetAttribute(k_layer1_tc<Tin, kPair>, cudaFuncAttributeMaxDynamicSharedMemorySize, k1Smem));
+        HB_CUDA(cudaFuncSetAttribute(k_layer1_tc<Tin, kPair, kMask>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     k1Smem));
         attr = true;
     }
     const long tiles = (long)g.nb * ((g.nx + k1X - 1) / k1X) * ((g.ny + k1Y - 1) / k1Y) * ((g.nz + k1Z - 1) / k1Z);
     const long cap = (long)k1CtasPerSm * sm_count();
     const int grid = (int)(tiles < cap ? tiles : cap);
-    HB_CUDA(launch_pdl_net(k_layer1_tc<Tin, kPair>, dim3(grid), dim3(k1Threads), (size_t)k1Smem, s, g, in, w1, a1,
-                           status));
+    HB_CUDA(launch_pdl_net(k_layer1_tc<Tin, kPair, kMask>, dim3(grid), dim3(k1Threads), (size_t)k1Smem, s, g, in, w1,
+                           (__nv_bfloat16*)a1, (const __nv_bfloat16*)act, status));
     return 0;
 }
 
 int launch_layer1_tc(const ConvGrid& g, const void* in, int in_f32, const float* w1, void* a1, int pair, int* status,
                      cudaStream_t s)
 {
-    auto* out = (__nv_bfloat16*)a1;
     if(in_f32)
-        return pair ? layer1_launch<float, true>(g, (const float*)in, w1, out, status, s)
-                    : layer1_launch<float, false>(g, (const float*)in, w1, out, status, s);
-    return pair ? layer1_launch<__nv_bfloat16, true>(g, (const __nv_bfloat16*)in, w1, out, status, s)
-                : layer1_launch<__nv_bfloat16, false>(g, (const __nv_bfloat16*)in, w1, out, status, s);
+        return pair ? layer1_launch<float, true>(g, (const float*)in, w1, a1, nullptr, status, s)
+                    : layer1_launch<float, false>(g, (const float*)in, w1, a1, nullptr, status, s);
+    return pair ? layer1_launch<__nv_bfloat16, true>(g, (const __nv_bfloat16*)in, w1, a1, nullptr, status, s)
+                : layer1_launch<__nv_bfloat16, false>(g, (const __nv_bfloat16*)in, w1, a1, nullptr, status, s);
+}
+
+int launch_layer3_grad(const ConvGrid& g, const float* gy, const float* w3, const void* a2, void* out, int pair,
+                       int* status, cudaStream_t s)
+{
+    return pair ? layer1_launch<float, true, true>(g, gy, w3, out, a2, status, s)
+                : layer1_launch<float, false, true>(g, gy, w3, out, a2, status, s);
 }
 
 int launch_odd_natural(long n, const float* y, float* out, cudaStream_t s)
@@ -1917,13 +1939,13 @@ int loss_parts(long points)
     return kLossBlocks;
 }
 
-int launch_loss_grad(const ConvGrid& g, const float* y, const float* e, float* d, const float* wnorm, float scale,
+int launch_loss_grad(const ConvGrid& g, float* y, const float* e, float* d, const float* wnorm, float scale,
                      int kind, int odd, void* G, float* loss_partial, cudaStream_t s)
 {
     const long n = g.points();
-    k_loss_diff<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, y, e, odd, d);
+    k_loss_diff<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, y, e, d);
     HB_LAUNCHED();
-    k_loss_grad<<<kLossBlocks, 256, 0, s>>>(g, d, wnorm, scale, kind, odd, (__nv_bfloat16*)G, loss_partial);
+    k_loss_grad<<<kLossBlocks, 256, 0, s>>>(g, d, wnorm, scale, kind, odd, (__nv_bfloat16*)G, y, loss_partial);
     HB_LAUNCHED();
     return 0;
 }

@@ -57,10 +57,14 @@ int launch_embed_scalar_level(const PermMap& pm, int nz, int ny, int nx, const f
                               const float* diag32, void* s1, cudaStream_t s);
 // a1 = bf16(relu(conv(in, W1))) from a scalar field in (FP32 when in_f32, else
 // BF16), 16 channels; pair: also the branch of -in at a1 + 16 * points.  The
-// 27 taps are the K dimension (im2col rows built in shared memory), the 16
-// channels N; `status` receives the code of a wait that gave up.
+// 27 taps are the K dimension, the 16 channels N; a1 is 32-byte aligned;
+// `status` receives the code of a wait that gave up.
 int launch_layer1_tc(const ConvGrid& g, const void* in, int in_f32, const float* w1, void* a1, int pair, int* status,
                      cudaStream_t s);
+// out = bf16(conv(gy, W3^T)) where a2 > 0: dL/da2 from dL/dy, one value a point;
+// pair: the second branch's dL/dy is -gy, its points follow in a2 and out.
+int launch_layer3_grad(const ConvGrid& g, const float* gy, const float* w3, const void* a2, void* out, int pair,
+                       int* status, cudaStream_t s);
 // Channel 0 of conv(a2, W3), odd-combined when pair ((y(a2) - y(a2 + 16 n)) / 2);
 // mode 0: set, 1: add into a level vector through pm (g.nb == 1); 2: natural out.
 // The 27 taps are stacked in N (one MMA row per staged input point gives its
@@ -104,12 +108,13 @@ int launch_normal_rhs(long long m, unsigned long long seed, const int* perm, dou
                       cudaStream_t s);
 
 // Loss of a batch: sum_b d_b.M d_b * wnorm[b] * scale with d = y - e (y the
-// odd part (y[p] - y[p+n])/2 when odd), M = I (kind 0) or the stencil A
+// odd evaluation's result when odd), M = I (kind 0) or the stencil A
 // (kind 1), as per-block partial sums (`loss_partial`, loss_parts(points)
 // floats), and its gradient 2 M d wnorm scale as BF16 channel 0 of G (odd:
-// +/- half for the two branches).  d: scratch of g.points() floats.
+// +/- half for the two branches) and, the first branch's, in place of y.
+// d: scratch of g.points() floats.
 int loss_parts(long points);
-int launch_loss_grad(const ConvGrid& g, const float* y, const float* e, float* d, const float* wnorm, float scale,
+int launch_loss_grad(const ConvGrid& g, float* y, const float* e, float* d, const float* wnorm, float scale,
                      int kind, int odd, void* G, float* loss_partial, cudaStream_t s);
 
 // Projects the weights (3 layers back to back) onto the tied odd form

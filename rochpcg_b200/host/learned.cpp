@@ -73,7 +73,7 @@ void smoother_reserve(Smoother& S, long points, bool training)
         S.a0 = dalloc<uint4>((size_t)points * br * 2);
         S.a1 = dalloc<uint4>((size_t)points * br * 2);
         S.a2 = dalloc<uint4>((size_t)points * br * 2);
-        S.y = dalloc<float>((size_t)points * br);
+        S.y = dalloc<float>((size_t)points);
         S.cap = points;
         S.epoch += 1;  // solve graphs that captured the old buffers are stale
     }
@@ -154,17 +154,6 @@ int smoother_level_apply(Smoother& S, const LevelOpt& o, const float* r, float* 
                                 S.status, s);
 }
 
-// Raw network output of a batch into y (both branches, 2 g.nb samples, when odd).
-static int forward_batch(Smoother& S, const hb::ConvGrid& g, const float* r, float* y, cudaStream_t s)
-{
-    const hb::ConvGrid gg{S.odd ? 2 * g.nb : g.nb, g.nz, g.ny, g.nx};
-    HB_RETURN_IF(smoother_prepare(S, s));
-    HB_RETURN_IF(hb::launch_embed_f32(g.points(), r, S.a0, S.odd ? 1 : 0, s));
-    HB_RETURN_IF(hb::launch_conv16(gg, S.a0, tiles(S, 0), hb::kOutReluBf16, S.a1, nullptr, nullptr, S.status, s));
-    HB_RETURN_IF(hb::launch_conv16(gg, S.a1, tiles(S, 1), hb::kOutReluBf16, S.a2, nullptr, nullptr, S.status, s));
-    return hb::launch_conv16(gg, S.a2, tiles(S, 2), hb::kOutF32C0, y, nullptr, nullptr, S.status, s);
-}
-
 // Evaluation as in the V-cycle (the one-channel forms of layers 1 and 3).
 int smoother_forward(Smoother& S, const hb::ConvGrid& g, const float* r, float* y, cudaStream_t s)
 {
@@ -180,7 +169,8 @@ int smoother_loss_grad(Smoother& S, const hb::ConvGrid& g0, const float* r, cons
                        float scale, int kind, cudaStream_t s)
 {
     smoother_reserve(S, g0.points(), true);
-    HB_RETURN_IF(forward_batch(S, g0, r, S.y, s));
+    HB_RETURN_IF(hb::launch_embed_f32(g0.points(), r, S.a0, S.odd ? 1 : 0, s));
+    HB_RETURN_IF(smoother_forward(S, g0, r, S.y, s));
     HB_RETURN_IF(hb::launch_loss_grad(g0, S.y, e, S.dbuf, wnorm, scale, kind, S.odd ? 1 : 0, S.g, S.loss_partial, s));
     HB_RETURN_IF(hb::launch_loss_accumulate(S.loss_partial, S.loss_acc, s));
     const hb::ConvGrid g{S.odd ? 2 * g0.nb : g0.nb, g0.nz, g0.ny, g0.nx};
@@ -189,7 +179,7 @@ int smoother_loss_grad(Smoother& S, const hb::ConvGrid& g0, const float* r, cons
     float* dw3 = S.dw + 2 * hb::kNetLayerWeights;
     // layer 3: dW3 = a2 (x) G; dL/da2 = conv(G, W3^T) where a2 > 0
     HB_RETURN_IF(hb::launch_conv16_wgrad(g, S.a2, S.g, S.partial, dw3, S.status, s));
-    HB_RETURN_IF(hb::launch_conv16(g, S.g, tiles_t(S, 2), hb::kOutMaskBf16, S.d, S.a2, nullptr, S.status, s));
+    HB_RETURN_IF(hb::launch_layer3_grad(g0, S.y, S.w + 2 * hb::kNetLayerWeights, S.a2, S.d, S.odd ? 1 : 0, S.status, s));
     // layer 2
     HB_RETURN_IF(hb::launch_conv16_wgrad(g, S.a1, S.d, S.partial, dw2, S.status, s));
     HB_RETURN_IF(hb::launch_conv16(g, S.d, tiles_t(S, 1), hb::kOutMaskBf16, S.g, S.a1, nullptr, S.status, s));
