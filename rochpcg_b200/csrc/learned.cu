@@ -914,17 +914,18 @@ __global__ void __launch_bounds__(k3Threads, 1)
 // point) a descriptor's K direction runs along x, and its M (N) direction steps
 // uniformly over (line, half): one MMA multiplies five lines of the input (M =
 // (line, channel), 80 of 128 rows used, the rest reads the bytes behind and is
-// ignored) with three lines of the gradient (N = (line, channel) = 48) over 16 x,
-// for one (dz, dx): the plane and the start x of A.  The nine (dz, dx)
-// accumulators take 432 TMEM columns; the (line, line) pairs one apart are
-// the dy taps, summed at the end.  A CTA walks units of 3 lines x 16 x x 8
-// planes: eight warps fetch units into a ring of three stages, a ninth issues the
-// MMAs from one elected lane (72 a unit, 40 cycles each; issued by a loader thread
-// between two block barriers they took 53, and loads and MMAs met at each unit).
-// A training batch of 64 samples of 16^3 (three weight gradients, two
-// convolutions): im2col 1572 us, bricks 361, with the warps' split 299
-// (289 with the forward passes' carried coordinates, 266 with the one-channel
-// forms of layers 1 and 3 in the forward pass and of layer 3's gradient).
+// ignored) with the three lines of each gradient plane it meets (N = (plane,
+// line, channel) = 144) over 16 x, for one dx: the start x of A.  The three column
+// blocks of a dx are the dz taps, the (line, line) pairs one apart the dy taps,
+// summed at the end; the nine blocks take 432 TMEM columns.  (One MMA per (dz, dx)
+// with N = 48 takes 53 cycles, N = 144 takes 75: 3800 -> 2000 cycles a unit.)  A
+// CTA walks units of 3 lines x 16 x x 8 planes: eight warps fetch units into a
+// ring of three stages, two units on their way in registers (one: 2600 cycles a
+// unit, the bound with this plan; cp.async straight into the ring was slower
+// still, 5000), a ninth issues the MMAs from one elected lane.  2 x 64 samples of
+// 16^3, with the reduction: 41.6 -> 33.4 us, four times as many 104 -> 77.  A
+// gradient step of 64 samples: im2col 1572 us, bricks 361, with the warps' split
+// 299, 266 with the one-channel forms of layers 1 and 3, with this plan 244.
 constexpr int kWgX = 16, kWgLines = 3, kWgZ = 8;                  // gradient points of a unit
 constexpr int kWgXA = kWgX + 2, kWgLinesA = kWgLines + 2, kWgZA = kWgZ + 2;  // input points, with the halo
 constexpr int kWgRowA = kWgXA * 16, kWgRowB = kWgX * 16;          // bytes of one line of one half
@@ -936,6 +937,7 @@ constexpr int kWgThreads = 256;                                   // loaders (an
 constexpr int kWgItemsA = kWgZA * kWgLinesA * kWgXA * 2, kWgItemsB = kWgZ * kWgLines * kWgX * 2;  // 16 B each
 constexpr int kWgLoadsA = (kWgItemsA + kWgThreads - 1) / kWgThreads;
 constexpr int kWgLoadsB = (kWgItemsB + kWgThreads - 1) / kWgThreads;
+constexpr int kWgLoads = kWgLoadsA + kWgLoadsB;
 constexpr int kWgStages = 3;
 constexpr int kWgSmem = kWgStages * kWgStage + 128;
 static_assert(9 * kWgN <= 512 && kWgStage % 128 == 0, "accumulators and stages");
@@ -988,67 +990,71 @@ __global__ void __launch_bounds__(kWgThreads + 32, 1)
 
     if(tid < kWgThreads)
     {
-        // ---- loaders: 16-byte items of unit u (plane, line, x, half), zero outside the sample
-        uint4 va[kWgLoadsA], vb[kWgLoadsB];
-        BrickWalk walk(g, kWgX, kWgLines, kWgZ, blockIdx.x, gridDim.x);
-        auto load = [&] {
-            const Brick bk = walk.at(kWgX, kWgLines, kWgZ);
-            const long b = bk.b;
-            const int x0 = bk.x0, y0 = bk.y0, z0 = bk.z0;
-            auto fetch = [&](const __nv_bfloat16* src, int z, int y, int xx, int half) {
-                if((unsigned)z >= (unsigned)g.nz || (unsigned)y >= (unsigned)g.ny || (unsigned)xx >= (unsigned)g.nx)
-                    return make_uint4(0, 0, 0, 0);
-                return __ldg(
-                    reinterpret_cast<const uint4*>(src + (((b * g.nz + z) * g.ny + y) * g.nx + xx) * kNetCh) + half);
-            };
+        // ---- loaders: a thread's 16-byte items (plane, line, x, half) are the same in every
+        // unit; zero outside the sample.  Two units are on their way in registers.
+        long at[kWgLoads];  // element, from the halo's corner
+        int to[kWgLoads], where[kWgLoads];  // byte of the stage; x | y << 8 | z << 16
 #pragma unroll
-            for(int k = 0; k < kWgLoadsA; ++k)
-            {
-                const int i = tid + k * kWgThreads, q = i >> 1, line = q / kWgXA;
-                va[k] = i < kWgItemsA ? fetch(x, z0 - 1 + line / kWgLinesA, y0 - 1 + line % kWgLinesA,
-                                              x0 - 1 + q % kWgXA, i & 1)
-                                      : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for(int k = 0; k < kWgLoadsB; ++k)
-            {
-                const int i = tid + k * kWgThreads, q = i >> 1, line = q / kWgX;
-                vb[k] = i < kWgItemsB ? fetch(gr, z0 + line / kWgLines, y0 + line % kWgLines, x0 + q % kWgX, i & 1)
-                                      : make_uint4(0, 0, 0, 0);
-            }
-        };
-        load();
-        int k = 0;
-        for(long u = blockIdx.x; u < U.count; u += gridDim.x, ++k)
+        for(int j = 0; j < kWgLoads; ++j)
         {
+            const bool in_a = j < kWgLoadsA;
+            const int i = tid + (in_a ? j : j - kWgLoadsA) * kWgThreads, q = i >> 1, half = i & 1;
+            const int wide = in_a ? kWgXA : kWgX, lines = in_a ? kWgLinesA : kWgLines, halo = in_a ? 0 : 1;
+            const int line = q / wide, px = q % wide + halo, py = line % lines + halo, pz = line / lines + halo;
+            to[j] = i >= (in_a ? kWgItemsA : kWgItemsB)
+                        ? -1
+                        : (in_a ? 0 : kWgOffB) + (line * 2 + half) * (in_a ? kWgRowA : kWgRowB) + q % wide * 16;
+            where[j] = px | py << 8 | pz << 16;
+            at[j] = (((long)pz * g.ny + py) * g.nx + px) * kNetCh + half * 8;
+        }
+        BrickWalk walk(g, kWgX, kWgLines, kWgZ, blockIdx.x, gridDim.x);
+        long next = blockIdx.x;  // unit the walk is at
+        auto load = [&](uint4 (&v)[kWgLoads]) {
+            if(next >= U.count) return;
+            const Brick bk = walk.at(kWgX, kWgLines, kWgZ);
+            const long corner =
+                ((((long)bk.b * g.nz + bk.z0 - 1) * g.ny + bk.y0 - 1) * g.nx + bk.x0 - 1) * kNetCh;
+#pragma unroll
+            for(int j = 0; j < kWgLoads; ++j)
+            {
+                const int xx = bk.x0 - 1 + (where[j] & 255), y = bk.y0 - 1 + (where[j] >> 8 & 255),
+                          z = bk.z0 - 1 + (where[j] >> 16);
+                const bool in = to[j] >= 0 && (unsigned)xx < (unsigned)g.nx && (unsigned)y < (unsigned)g.ny &&
+                                (unsigned)z < (unsigned)g.nz;
+                v[j] = make_uint4(0, 0, 0, 0);
+                if(in) v[j] = __ldg(reinterpret_cast<const uint4*>((j < kWgLoadsA ? x : gr) + corner + at[j]));
+            }
+            walk.next();
+            next += gridDim.x;
+        };
+        int k = 0;
+        // unit k from v into its stage, then unit k + 2 on its way into v
+        auto step = [&](uint4 (&v)[kWgLoads]) {
             const int st = k % kWgStages;
             // the MMAs that read this stage kWgStages units ago
-            if(!role_wait(&empty[st], (uint32_t)((k / kWgStages) & 1) ^ 1u, abort_flag, status, 2)) break;
+            if(!role_wait(&empty[st], (uint32_t)((k / kWgStages) & 1) ^ 1u, abort_flag, status, 2)) return false;
             unsigned char* sA = smem + st * kWgStage;
 #pragma unroll
-            for(int j = 0; j < kWgLoadsA; ++j)
-            {
-                const int i = tid + j * kWgThreads, q = i >> 1, line = q / kWgXA;
-                if(i < kWgItemsA)
-                    *reinterpret_cast<uint4*>(sA + (line * 2 + (i & 1)) * kWgRowA + q % kWgXA * 16) = va[j];
-            }
-#pragma unroll
-            for(int j = 0; j < kWgLoadsB; ++j)
-            {
-                const int i = tid + j * kWgThreads, q = i >> 1, line = q / kWgX;
-                if(i < kWgItemsB)
-                    *reinterpret_cast<uint4*>(sA + kWgOffB + (line * 2 + (i & 1)) * kWgRowB + q % kWgX * 16) = vb[j];
-            }
+            for(int j = 0; j < kWgLoads; ++j)
+                if(to[j] >= 0) *reinterpret_cast<uint4*>(sA + to[j]) = v[j];
             fence_async_smem();
             mbar_arrive(&full[st]);
-            walk.next();
-            if(u + gridDim.x < U.count) load();
+            load(v);
+            ++k;
+            return true;
+        };
+        uint4 even[kWgLoads], odd[kWgLoads];
+        load(even);
+        load(odd);
+        for(long u = blockIdx.x; u < U.count; u += 2 * (long)gridDim.x)
+        {
+            if(!step(even)) break;
+            if(u + gridDim.x < U.count && !step(odd)) break;
         }
     }
     else
     {
         // ---- MMA issuer: the whole warp walks the loop, one elected lane issues
-        constexpr uint32_t idesc = umma_idesc_bf16(128, kWgN, true, true);
         int k = 0;
         for(long u = blockIdx.x; u < U.count; u += gridDim.x, ++k)
         {
@@ -1060,13 +1066,20 @@ __global__ void __launch_bounds__(kWgThreads + 32, 1)
             const uint64_t bd = umma_desc(smem_u32(smem + st * kWgStage + kWgOffB), 128, kWgRowB);
             if(elect_one())
             {
-#pragma unroll 1
-                for(int z = 0; z < kWgZ; ++z)
+                // input plane q meets gradient planes q - 2 .. q, column block j the
+                // plane q - 2 + j (dz = 1 - j); a plane with all three goes first, it
+                // starts the accumulators
 #pragma unroll
-                    for(int t = 0; t < 9; ++t)
-                        mma_bf16(tmem + (uint32_t)(t * kWgN),
-                                 ad + (uint64_t)(((z + t / 3) * kWgPlaneA + t % 3 * 16) >> 4),
-                                 bd + (uint64_t)((z * kWgPlaneB) >> 4), idesc, (k == 0 && z == 0) ? 0u : 1u);
+                for(int i = 0; i < kWgZA; ++i)
+                {
+                    const int q = (i + 2) % kWgZA;
+                    const int lo = q < 2 ? 2 - q : 0, hi = q > kWgZ - 1 ? kWgZ + 1 - q : 2;
+                    const uint32_t idesc = umma_idesc_bf16(128, (hi - lo + 1) * kWgN, true, true);
+#pragma unroll
+                    for(int t = 0; t < 3; ++t)
+                        mma_bf16(tmem + (uint32_t)((3 * t + lo) * kWgN), ad + (uint64_t)((q * kWgPlaneA + t * 16) >> 4),
+                                 bd + (uint64_t)(((q - 2 + lo) * kWgPlaneB) >> 4), idesc, (k == 0 && i == 0) ? 0u : 1u);
+                }
                 mma_commit(&empty[st]);
             }
             __syncwarp();
@@ -1093,7 +1106,9 @@ __global__ void __launch_bounds__(kWgThreads + 32, 1)
             for(int t = 0; t < 9; ++t)
             {
                 float v[16];
-                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(t * kWgN + r * kNetCh), v);
+                // t = 3 (dz + 1) + (dx + 1)
+                const int block = 3 * (t % 3) + 2 - t / 3;
+                tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(block * kWgN + r * kNetCh), v);
                 if(yy < kWgLinesA && dy >= -1 && dy <= 1)
                 {
                     // [tap][co][ci]: the lanes of a line on consecutive words
