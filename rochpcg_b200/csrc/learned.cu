@@ -1,33 +1,26 @@
 // Learned smoother kernels on the 5th-generation tensor cores (tcgen05).  No
 // reference counterpart: the conv-net smoother is new in this library.
 //
-// Forward / input-gradient convolution (k_conv16).  Every layer runs as a
-// 16 -> 16 channel 3x3x3 convolution (layer 1 has one real input channel and
-// layer 3 one real output channel, the other weights are zero), so one kernel
-// serves the forward pass and the input gradient (the transposed convolution
-// is a convolution with mirrored taps and swapped channels).  A CTA owns a
-// brick of 16 x 8 x 2 points = two 128-row M tiles (one per z plane) and
-// stages the brick's halo once, as three copies shifted by dx = -1, 0, +1.
-// Each copy keeps one 16-byte row (8 BF16 channels) per point, the two
-// channel halves in separate regions, so in the no-swizzle K-major operand
-// layout every 8-row core matrix is contiguous and consecutive rows are 16
-// bytes apart.  A tap (dz, dy, dx) is then only a start-address offset into
-// copy dx: 27 taps x 2 tiles = 54 tcgen05.mma (M=128, N=16, K=16) accumulate
-// the brick's outputs in 32 TMEM columns, read back with tcgen05.ld.
+// Convolution (k_conv16).  16 -> 16 channels, 3x3x3: layer 2, and the gradient of
+// its input (the transposed convolution is a convolution with mirrored taps and
+// swapped channels).  Bricks of 14 x 8 x 4 points, the dx and dz taps stacked in
+// the MMA's N.  Layer 3 (k_layer3_tc, one output channel) is the same brick plan,
+// layer 1 (k_layer1_tc, one input channel, also the gradient of layer 3's input)
+// has the 27 taps as K.
 //
 // Weight gradient (k_conv16_wgrad).  dW[tap][ci][co] = sum_p x[p+tap][ci] *
 // g[p][co] is a GEMM over points with both operands MN-major (8 channels = one
 // 16-byte core-matrix row): M = (input line, input channel), N = (gradient
-// line, output channel), K = 16 points along x, one accumulator per (dz, dx).
-// Per-CTA partial sums are reduced in a fixed order, so the gradient is
+// plane, line, output channel), K = 16 points along x, one accumulator per dx and
+// plane.  Per-CTA partial sums are reduced in a fixed order, so the gradient is
 // deterministic.
 //
-// Operand layouts are the canonical no-swizzle ("interleaved") forms, in
+// Operand layouts without a swizzle are the canonical "interleaved" forms, in
 // 16-byte units: K-major ((8,m),2):((1,SBO),LBO); MN-major
 // ((1,m),(8,k)):((.,SBO),(1,LBO)).
 //
-// Waits.  The only waits are on an mbarrier completed by tcgen05.commit; each
-// is bounded.  On timeout the CTA records an error in *status, waits once more
+// Waits.  All waits are on mbarriers (TMA, tcgen05.commit, the roles' arrivals);
+// each is bounded.  On timeout the CTA records an error in *status, waits once more
 // (bounded) for its MMAs, leaves its loop as a whole block and still frees its
 // TMEM, so the context stays usable.
 #include <cuda.h>

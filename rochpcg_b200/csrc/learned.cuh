@@ -67,9 +67,8 @@ int launch_layer3_grad(const ConvGrid& g, const float* gy, const float* w3, cons
                        int* status, cudaStream_t s);
 // Channel 0 of conv(a2, W3), odd-combined when pair ((y(a2) - y(a2 + 16 n)) / 2);
 // mode 0: set, 1: add into a level vector through pm (g.nb == 1); 2: natural out.
-// The 27 taps are stacked in N (one MMA row per staged input point gives its
-// contribution to each neighbour), the pair is folded into K, and the 27-tap
-// gather runs in the epilogue; `status` receives the code of a wait that gave up.
+// k_conv16's plan with one output channel, the pair folded into K; `status`
+// receives the code of a wait that gave up.
 int launch_layer3_tc(const ConvGrid& g, const PermMap* pm, const void* a2, const float* w3, int pair, int mode,
                      float* out, int* status, cudaStream_t s);
 
