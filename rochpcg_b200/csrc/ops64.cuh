@@ -46,10 +46,10 @@ ColorChunks make_chunks(int m, int ncolors, const int* offsets);
 // of its launch needs only some groups (the zero-guess sweeps of a colour, from
 // the colour's extreme diagonal positions) issues no instructions for the
 // others; the sum is the same, since the groups left out hold no slot of the
-// range.
-template <int GLO = 0, int GHI = kWidth / 9, typename ColPred>
+// range.  x: a pointer, or what reads x[i].
+template <int GLO = 0, int GHI = kWidth / 9, typename X, typename ColPred>
 __device__ __forceinline__ double ell_row_sum(int m, int row, const int* __restrict__ ell_col,
-                                              const double* __restrict__ ell_val, const double* x, double sum,
+                                              const double* __restrict__ ell_val, X x, double sum,
                                               double s, int p_lo, int p_hi, ColPred use_col)
 {
     constexpr int G = 9;

@@ -17,10 +17,12 @@
 // one-launch kernels: the same sums, bit for bit.
 //
 // A zero-guess step in a graph, one cluster against 15 launches: 16^3 FP32 18.6
-// against 26.8 us, FP64 20.6 against 32.8, ELL values 20.6 against 42.5; 32^3 20.6
-// / 30.8, 22.6 / 36.9, 24.6 / 45.1.  The whole V-cycle called through the
-// operator API: 16^3 FP64 446 -> 151 us, 104^3 mixed 466 -> 334 us.
+// against 26.8 us, FP64 20.6 against 32.8, ELL arrays 20.5 against 42.5; 32^3 20.6
+// / 30.8, 22.6 / 36.9, 30.7 / 45.1 (the check of 27 slots a row is 8 us of it).
+// The whole V-cycle called through the operator API: 16^3 FP64 446 -> 137 us,
+// 104^3 mixed 466 -> 334 us.
 #include <algorithm>
+#include <type_traits>
 
 #include "small_level.cuh"
 
@@ -32,7 +34,7 @@ constexpr int kMaxCtas = 16;
 // A thread has one row of each colour, so a level fits where a CTA's share of a
 // pass does: 640 threads leave 96 registers (48 x 24 x 40 with 576 gains, 28.3
 // against 31.3 us; two rows a thread at 40^3 lost, 40.4 against 32.8 us), the
-// ELL form needs 128.
+// ELL form needs 112 and always takes its 512, which read the arrays.
 constexpr int kMaxThreads = 640, kMaxThreadsEll = 512;
 constexpr int kSmallSmem = 220 * 1024;
 constexpr int kOneCta = 2048;    // rows of a level up to which one CTA takes it: no cluster barrier (8^3 20.5 -> 14.5 us)
@@ -92,11 +94,42 @@ struct SmallArgs
     T* r;
     T* x;
     double* z64;
-    const double* val;     // ELL values, slot p of row i at p*m + i
     const int* inj_c;      // coarse row of each row of colour 7
     T* rc;                 // coarse residual (may be null)
     Prolong<T> pro;
 };
+
+// What the ELL form reads besides.
+struct EllArgs
+{
+    SmallEll m;
+    int rows;              // rows of a pass and CTA at most, a multiple of 32
+    int dcol[8][27];       // by stencil point: its column in a row of a colour, from the row's brick position
+    signed char slot[8][27];  // and its slot
+};
+
+struct NoEll
+{
+};
+
+// The columns as they are at set-up: stencil point t of a colour-v row at brick
+// position (kx, ky, kz) is dcol[v][t] + (kz * by + ky) * bx + kx with the extents
+// of the neighbour's brick.
+void expected_columns(const StencilLevel& L, EllArgs* e)
+{
+    constexpr Order o = make_order();
+    for(int v = 0; v < 8; ++v)
+        for(int j = 0; j < 27; ++j)
+        {
+            const int cls = o.cls[v], dx = o.dx[v][j], dy = o.dy[v][j], dz = o.dz[v][j];
+            const int c = colour_of(cls ^ (((dx & 1) << 2) | ((dy & 1) << 1) | (dz & 1)));
+            auto shift = [](int parity, int d) { return parity + d < 0 ? -1 : (parity + d > 1 ? 1 : 0); };
+            const int sx = shift((cls >> 2) & 1, dx), sy = shift((cls >> 1) & 1, dy), sz = shift(cls & 1, dz);
+            const int t = (dz + 1) * 9 + (dy + 1) * 3 + dx + 1;
+            e->dcol[v][t] = L.offsets[c] + (sz * L.by[c] + sy) * L.bx[c] + sx;
+            e->slot[v][t] = (signed char)j;
+        }
+}
 
 __device__ __forceinline__ unsigned cluster_rank()
 {
@@ -131,6 +164,16 @@ __device__ __forceinline__ void store_peer(float* cell, unsigned rank, float v)
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(p), "f"(v) : "memory");
 }
 
+// the int cell of CTA `rank` of the cluster
+__device__ __forceinline__ int load_peer(const int* cell, unsigned rank)
+{
+    unsigned a = (unsigned)__cvta_generic_to_shared(cell), p;
+    int v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(p) : "r"(a), "r"(rank));
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
+    return v;
+}
+
 __device__ __forceinline__ float mul_once(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_once(double a, double b) { return __dmul_rn(a, b); }
 
@@ -146,28 +189,55 @@ __device__ __forceinline__ void finish(const SmallArgs<T>& a, int g, T v)
     a.pro.add(g, v);
 }
 
-__device__ const double d_minus_one = -1.0;
+// x of a level through L2: in the passes on any matrix other CTAs write it.
+struct L2Reads
+{
+    const double* x;
+    __device__ __forceinline__ double operator[](int i) const { return __ldcg(x + i); }
+};
+
+// The row of a full step, of a zero-guess step's forward pass (offset: the
+// colour's first row) or its backward pass on any matrix: k_symgs_sweep,
+// k_symgs_fwd0 and k_symgs_bwd0.
+template <bool kZero>
+__device__ double any_row(const SmallArgs<double>& a, const SmallEll& e, int row, int offset, bool back)
+{
+    const int m = a.m;
+    const L2Reads x{a.x};
+    double sum;
+    if constexpr(!kZero)
+        sum = ell_row_sum(m, row, e.col, e.val, x, a.r[row], -1.0, 0, kWidth,
+                          [m, row](int col) { return col >= 0 && col < m && col != row; });
+    else if(!back)
+        sum = ell_row_sum(m, row, e.col, e.val, x, a.r[row], -1.0, 0, offset > 0 ? e.diag_idx[row] : 0,
+                          [offset](int col) { return col >= 0 && col < offset; });
+    else
+        sum = ell_row_sum(m, row, e.col, e.val, x, __dmul_rn(x[row], a.diag[row]), -1.0, e.diag_idx[row] + 1, kWidth,
+                          [offset, m](int col) { return col >= offset && col < m; });
+    return sum * a.inv_diag[row];
+}
 
 // The dynamic shared memory: the x bricks, then per colour and thread the
-// row's r, 1/a_ii and (zero guess) a_ii, its cell, and with the ELL values the
-// slots its faces remove.
-template <typename T, bool kZero, bool kEll>
-constexpr size_t bytes_per_thread = 8 * ((kZero ? 3 : 2) * sizeof(T) + 4 + (kEll ? 4 : 0));
+// row's r, 1/a_ii and (zero guess) a_ii, and its cell.
+template <typename T, bool kZero>
+constexpr size_t bytes_per_thread = 8 * ((kZero ? 3 : 2) * sizeof(T) + 4);
 
 // s_cell: the row's cell, or kNone; flags where its value has a copy in the CTA below or above
 constexpr int kNone = -1, kToBelow = 1 << 30, kToAbove = 1 << 29, kCellMask = kToAbove - 1;
 
 // kZero: the zero-guess step (forward pass: slots before the diagonal,
 // backward: a_ii x_i and the slots after it) and, with rc given, the
-// restriction of its residual; else the full step.  kEll: the slots' values
-// are read -- once, by the row's thread before the first pass; where a CTA's
-// are all -1 its passes are the implicit ones (sum + x is fma(1, x, sum)), else
-// every pass reads them again.  A thread has at most one row of each colour; what
-// a pass needs of it besides its neighbours' x is fetched between the
-// barrier's arrival and its wait.
+// restriction of its residual; else the full step.  kEll: the step is that of
+// the ELL arrays as they are now -- they are read once, before the first pass.
+// Where every column, value and diagonal slot of the cluster's rows is the
+// stencil's, the passes are the implicit ones (sum + x is fma(1, x, sum)); else
+// the cluster runs them on the arrays, with x in global memory.  A thread has at most one row of each colour; what a pass needs of it
+// besides its neighbours' x is fetched between the barrier's arrival and its
+// wait.
 template <typename T, bool kZero, bool kEll>
 __global__ void __launch_bounds__(kEll ? kMaxThreadsEll : kMaxThreads, 1)
-    k_small_symgs(const __grid_constant__ SmallArgs<T> a)
+    k_small_symgs(const __grid_constant__ SmallArgs<T> a,
+                  const __grid_constant__ std::conditional_t<kEll, EllArgs, NoEll> ell)
 {
     extern __shared__ __align__(16) unsigned char small_smem[];
     const int nt = blockDim.x, tid = threadIdx.x;
@@ -176,10 +246,10 @@ __global__ void __launch_bounds__(kEll ? kMaxThreadsEll : kMaxThreads, 1)
     T* const s_inv = s_r + 8 * nt;
     T* const s_diag = s_inv + 8 * nt;  // kZero only
     int* const s_cell = reinterpret_cast<int*>(xs + 8 * a.brick + (kZero ? 24 : 16) * nt) + tid;
-    int* const s_gone = s_cell + 8 * nt;
     __shared__ __align__(16) int s_tab[8][28];  // per colour: cell offset of each slot but the diagonal's, in order
     __shared__ int s_row0[8];                   // per colour: the CTA's first row
     __shared__ int s_dp[8];                     // per colour: the diagonal's slot
+    __shared__ int s_other;                     // kEll: some row of this CTA is not the stencil's
     const unsigned rank = cluster_rank(), size = cluster_size();
     const int p0 = (int)(rank * (unsigned)a.pairs / size), p1 = (int)((rank + 1) * (unsigned)a.pairs / size);
     const int np = p1 - p0;
@@ -194,7 +264,7 @@ __global__ void __launch_bounds__(kEll ? kMaxThreadsEll : kMaxThreads, 1)
     auto quotient = [](int t, int n) { return __float2int_rd(((float)t + 0.5f) * __frcp_rn((float)n)); };
 
     // this thread's row of every colour
-    bool plain = true;
+    unsigned other = 0;  // kEll: bits in which rows differ from the stencil's
 #pragma unroll
     for(int v = 0; v < 8; ++v)
     {
@@ -224,20 +294,50 @@ __global__ void __launch_bounds__(kEll ? kMaxThreadsEll : kMaxThreads, 1)
         }
         else r = __ldg(a.r + g);
         s_r[v * nt] = r;
-        if constexpr(kEll)
+    }
+    if constexpr(kEll)
+    {
+        // All threads of a full block, a row of some colour each (by the rows' own
+        // threads, unrolled over the colours: 16^3 V-cycle 133 -> 205 us).
+#pragma unroll 1
+        for(int e = tid; e < 8 * ell.rows; e += nt)
         {
-            const int ix = 2 * kx + px, iy = 2 * ky + py, iz = 2 * (p0 + kp) + pz;
-            const unsigned gone = (ix == 0 ? o.gone[v][0] : 0u) | (ix == a.nx - 1 ? o.gone[v][1] : 0u) |
-                                  (iy == 0 ? o.gone[v][2] : 0u) | (iy == a.ny - 1 ? o.gone[v][3] : 0u) |
-                                  (iz == 0 ? o.gone[v][4] : 0u) | (iz == a.nz - 1 ? o.gone[v][5] : 0u);
-            s_gone[v * nt] = (int)gone;
-            // the row's slots, packed; the diagonal's is not looked at
-            const int mine = o.dp[v] - __popc(gone & ((1u << o.dp[v]) - 1u)), slots = 27 - __popc(gone);
+            const int v = e / ell.rows, t = e - v * ell.rows;
+            const int cls = c_order.cls[v], px = (cls >> 2) & 1, py = (cls >> 1) & 1, pz = cls & 1;
+            const int bx = (a.nx - px + 1) / 2, by = (a.ny - py + 1) / 2, bz = (a.nz - pz + 1) / 2;
+            if(t >= (min(p1, bz) - p0) * by * bx) continue;
+            const int q = quotient(t, bx), kx = t - q * bx, kp = quotient(q, by), ky = q - kp * by, kz = p0 + kp;
+            const int g = a.off[v] + p0 * by * bx + t;
+            const int ix = 2 * kx + px, iy = 2 * ky + py, iz = 2 * kz + pz;
+            const unsigned* face = c_order.gone[v];
+            const unsigned gone = (ix == 0 ? face[0] : 0u) | (ix == a.nx - 1 ? face[1] : 0u) |
+                                  (iy == 0 ? face[2] : 0u) | (iy == a.ny - 1 ? face[3] : 0u) |
+                                  (iz == 0 ? face[4] : 0u) | (iz == a.nz - 1 ? face[5] : 0u);
+            // the row's position in the neighbours' bricks: index bit 0 dx odd, bit 1 dy odd
+            int at[4];
 #pragma unroll
-            for(int p = 0; p < 27; ++p)
+            for(int k = 0; k < 4; ++k)
+                at[k] = (kz * ((a.ny + 1 - (py ^ (k >> 1))) / 2) + ky) * ((a.nx + 1 - (px ^ (k & 1))) / 2) + kx;
+            const double diag = kZero ? __ldg(a.diag + g) : 0.0;
+            // slots are packed: those the faces remove leave the row's last ones empty
+#pragma unroll
+            for(int n = 0; n < 27; ++n)
             {
-                const double w = __ldg(p < slots && p != mine ? a.val + (p * a.m + g) : &d_minus_one);
-                plain = plain && w == -1.0;
+                const int j = ell.slot[v][n], missing = __popc(gone & ((1u << j) - 1u));
+                const bool off = gone >> j & 1u;
+                const int at_e = (off ? 26 - missing : j - missing) * a.m + g;
+                const unsigned c = (unsigned)__ldg(ell.m.col + at_e);
+                const unsigned want = (unsigned)(at[(n % 3 != 1) + 2 * (n / 3 % 3 != 1)] + ell.dcol[v][n]);
+                unsigned differs = c ^ want;
+                if(n != 13 || kZero)
+                    differs |= __ldg(ell.m.val + at_e) == (n == 13 ? diag : -1.0) ? 0u : 1u;
+                other |= off ? (unsigned)(c < (unsigned)a.m) : differs;
+            }
+            if constexpr(kZero)
+            {
+                const int dp = c_order.dp[v];
+                other |= (unsigned)(__ldg(ell.m.diag_idx + g) ^ (dp - __popc(gone & ((1u << dp) - 1u))));
+                if(a.rc && v == 7) other |= (unsigned)(__ldg(ell.m.inj_f + (g - a.off[7])) ^ g);
             }
         }
     }
@@ -251,8 +351,12 @@ __global__ void __launch_bounds__(kEll ? kMaxThreadsEll : kMaxThreads, 1)
                 cell_of(hx + c_order.dx[v][j], hy + c_order.dy[v][j], hz + c_order.dz[v][j]) - cell_of(hx, hy, hz);
         else if(j == 27) s_tab[v][26] = s_tab[v][27] = 0;
     }
-    const bool ell = kEll && !__syncthreads_and(plain);
-    if constexpr(!kEll) __syncthreads();
+    if constexpr(kEll)
+    {
+        const int any = __syncthreads_or((int)other);
+        if(tid == 0) s_other = any;
+    }
+    else __syncthreads();
     if constexpr(!kZero)
     {
         for(int v = 0; v < 8; ++v)
@@ -303,6 +407,40 @@ __global__ void __launch_bounds__(kEll ? kMaxThreadsEll : kMaxThreads, 1)
     };
     fetch(0);
     wait();
+    if constexpr(kEll)
+    {
+        int any = s_other;
+        if(size > 1)
+        {
+            const int lane = tid & 31;
+            any = __any_sync(0xffffffffu, lane < (int)size ? load_peer(&s_other, (unsigned)lane) : 0);
+        }
+        if(any)
+        {
+#pragma unroll 1
+            for(int i = 0; i < 15; ++i)
+            {
+                const int v = colour(i);
+                if(s_cell[v * nt] != kNone)
+                {
+                    const int row = s_row0[v] + tid;
+                    const double out = any_row<kZero>(a, ell.m, row, a.off[v], i >= 8);
+                    a.x[row] = out;
+                    if(i >= 7) a.pro.add(row, out);
+                }
+                arrive();
+                wait();
+            }
+            if(!kZero || !a.rc) return;
+            for(int ic = (int)rank * nt + tid; ic < ell.m.nc; ic += (int)size * nt)
+            {
+                const int row = ell.m.inj_f[ic], m = a.m;
+                a.rc[a.inj_c[ic]] = ell_row_sum(m, row, ell.m.col, ell.m.val, L2Reads{a.x}, a.r[row], -1.0, 0, kWidth,
+                                                [m](int col) { return col >= 0 && col < m; });
+            }
+            return;
+        }
+    }
 #pragma unroll 1
     for(int i = 0; i < passes; ++i)
     {
@@ -324,32 +462,8 @@ __global__ void __launch_bounds__(kEll ? kMaxThreadsEll : kMaxThreads, 1)
 #pragma unroll
                 for(int e = 0; e < 26; ++e) nb[e] = e >= lo ? nb[e] : T(-0.0);
             }
-            if constexpr(kEll)
-            {
-                if(ell)
-                {
-                    const unsigned gone = (unsigned)s_gone[v * nt];
-                    const int dp = s_dp[v], g = s_row0[v] + tid;
-                    const int hi = kZero && i < 8 ? dp : 26;
-                    for(int e = lo; e < hi; ++e)
-                    {
-                        const int j = e + (e >= dp);
-                        if(gone >> j & 1u) continue;
-                        const int p = j - __popc(gone & ((1u << j) - 1u));
-                        sum = fma(-__ldg(a.val + (p * a.m + g)), own[s_tab[v][e]], sum);
-                    }
-                }
-                else
-                {
 #pragma unroll
-                    for(int e = 0; e < 26; ++e) sum = sum + nb[e];
-                }
-            }
-            else
-            {
-#pragma unroll
-                for(int e = 0; e < 26; ++e) sum = sum + nb[e];
-            }
+            for(int e = 0; e < 26; ++e) sum = sum + nb[e];
             if(kZero && i == 15)  // the diagonal is colour 7's last slot
                 a.rc[a.inj_c[s_row0[7] + tid - a.off[7]]] = fma_once(-opd, *own, sum);
             else
@@ -414,7 +528,8 @@ int max_ctas()
 // Cluster shape of a level.
 struct Shape
 {
-    int ctas, threads, per;  // per: z-plane pairs of a CTA at most
+    int ctas, per;      // z-plane pairs of a CTA at most
+    int rows, threads;  // rows of a pass and CTA at most, in whole warps
     size_t smem;
 };
 
@@ -429,9 +544,10 @@ Shape shape_of(const StencilLevel& L)
     while(s.ctas > pairs) s.ctas /= 2;
     s.per = (pairs + s.ctas - 1) / s.ctas;
     const int rows = ((L.nx + 1) / 2) * ((L.ny + 1) / 2) * s.per;
-    s.threads = (rows + 31) / 32 * 32;
+    s.rows = (rows + 31) / 32 * 32;
+    s.threads = kEll ? kMaxThreadsEll : s.rows;
     s.smem = sizeof(T) * 8 * (size_t)((L.nx + 3) / 2) * ((L.ny + 3) / 2) * (s.per + 1) +
-             bytes_per_thread<T, true, kEll> * (size_t)s.threads;
+             bytes_per_thread<T, true> * (size_t)s.threads;
     return s;
 }
 
@@ -451,10 +567,12 @@ SmallArgs<T> args_of(const StencilLevel& L)
 }
 
 template <typename T, bool kZero, bool kEll>
-int launch_shape(const StencilLevel& L, SmallArgs<T> a, cudaStream_t s)
+int launch_shape(const StencilLevel& L, SmallArgs<T> a, std::conditional_t<kEll, EllArgs, NoEll> ell,
+                 cudaStream_t s)
 {
     const Shape sh = shape_of<T, kEll>(L);
     a.brick = a.sx * a.sy * (sh.per + 1);
+    if constexpr(kEll) ell.rows = sh.rows;
     const auto kernel = k_small_symgs<T, kZero, kEll>;
     HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem));
     HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -470,16 +588,22 @@ int launch_shape(const StencilLevel& L, SmallArgs<T> a, cudaStream_t s)
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    HB_CUDA(cudaLaunchKernelEx(&cfg, kernel, a));
+    HB_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, ell));
     return 0;
 }
 
 template <typename T, bool kZero>
-int launch_small(const StencilLevel& L, const SmallArgs<T>& a, cudaStream_t s)
+int launch_small(const StencilLevel& L, const SmallArgs<T>& a, const SmallEll* ell, cudaStream_t s)
 {
     if constexpr(sizeof(T) == 8)
-        if(a.val) return launch_shape<T, kZero, true>(L, a, s);
-    return launch_shape<T, kZero, false>(L, a, s);
+        if(ell)
+        {
+            EllArgs e{};
+            e.m = *ell;
+            expected_columns(L, &e);
+            return launch_shape<T, kZero, true>(L, a, e, s);
+        }
+    return launch_shape<T, kZero, false>(L, a, NoEll{}, s);
 }
 
 }  // namespace
@@ -491,12 +615,12 @@ bool small_level_ok(const StencilLevel& L, bool ell)
     for(int p = 0; p < 8; ++p)
         if(L.color_of_par[p] != colour_of(p)) return false;
     const Shape s = ell ? shape_of<T, true>(L) : shape_of<T, false>(L);
-    return s.threads <= (ell ? kMaxThreadsEll : kMaxThreads) && s.smem <= kSmallSmem;
+    return s.rows <= (ell ? kMaxThreadsEll : kMaxThreads) && s.smem <= kSmallSmem;
 }
 
 template <typename T>
 int launch_small_zero(const StencilLevel& L, const T* diag, const T* inv_diag, const double* r64, T* r, T* x,
-                      const double* ell_val, const int* inj_c, T* rc, cudaStream_t s, Prolong<T> pro)
+                      const SmallEll* ell, const int* inj_c, T* rc, cudaStream_t s, Prolong<T> pro)
 {
     SmallArgs<T> a = args_of<T>(L);
     a.diag = diag;
@@ -506,34 +630,32 @@ int launch_small_zero(const StencilLevel& L, const T* diag, const T* inv_diag, c
     a.r64 = r64;
     a.r = r;
     a.x = x;
-    a.val = ell_val;
     a.pro = pro;
-    return launch_small<T, true>(L, a, s);
+    return launch_small<T, true>(L, a, ell, s);
 }
 
 template <typename T>
 int launch_small_symgs(const StencilLevel& L, const T* inv_diag, const T* r, T* x, double* z64,
-                       const double* ell_val, cudaStream_t s, Prolong<T> pro)
+                       const SmallEll* ell, cudaStream_t s, Prolong<T> pro)
 {
     SmallArgs<T> a = args_of<T>(L);
     a.inv_diag = inv_diag;
     a.r = const_cast<T*>(r);
     a.x = x;
     a.z64 = z64;
-    a.val = ell_val;
     a.pro = pro;
-    return launch_small<T, false>(L, a, s);
+    return launch_small<T, false>(L, a, ell, s);
 }
 
 template bool small_level_ok<float>(const StencilLevel&, bool);
 template bool small_level_ok<double>(const StencilLevel&, bool);
 template int launch_small_zero<float>(const StencilLevel&, const float*, const float*, const double*, float*, float*,
-                                      const double*, const int*, float*, cudaStream_t, Prolong<float>);
+                                      const SmallEll*, const int*, float*, cudaStream_t, Prolong<float>);
 template int launch_small_zero<double>(const StencilLevel&, const double*, const double*, const double*, double*,
-                                       double*, const double*, const int*, double*, cudaStream_t, Prolong<double>);
+                                       double*, const SmallEll*, const int*, double*, cudaStream_t, Prolong<double>);
 template int launch_small_symgs<float>(const StencilLevel&, const float*, const float*, float*, double*,
-                                       const double*, cudaStream_t, Prolong<float>);
+                                       const SmallEll*, cudaStream_t, Prolong<float>);
 template int launch_small_symgs<double>(const StencilLevel&, const double*, const double*, double*, double*,
-                                        const double*, cudaStream_t, Prolong<double>);
+                                        const SmallEll*, cudaStream_t, Prolong<double>);
 
 }  // namespace hb

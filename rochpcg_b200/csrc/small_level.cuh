@@ -5,6 +5,7 @@
 #pragma once
 
 #include "mixed.cuh"
+#include "ops64.cuh"
 
 namespace hb {
 
@@ -13,16 +14,28 @@ namespace hb {
 template <typename T>
 bool small_level_ok(const StencilLevel& L, bool ell);
 
+// The ELL arrays of a level (launch_symgs, launch_symgs_zero, launch_restrict):
+// the step is the one on their present contents, whatever was changed in them
+// since set-up.
+struct SmallEll
+{
+    const int* col;
+    const double* val;
+    const int* diag_idx;
+    const int* inj_f;  // with nc: the restriction's
+    int nc;
+};
+
 // One zero-guess step: x from r; r64 (float only, may be null): r comes in
-// FP64 and its float copy is stored in r.  ell_val: the level's ELL values
-// (double only; null: the stencil's -1).  rc (may be null): also the residual
+// FP64 and its float copy is stored in r.  ell (double only): the level's ELL
+// arrays; null: the verified stencil.  rc (may be null): also the residual
 // at the injected rows, rc[inj_c[i]] for row i of the parity-0 colour.
 template <typename T>
 int launch_small_zero(const StencilLevel& L, const T* diag, const T* inv_diag, const double* r64, T* r, T* x,
-                      const double* ell_val, const int* inj_c, T* rc, cudaStream_t s, Prolong<T> pro);
+                      const SmallEll* ell, const int* inj_c, T* rc, cudaStream_t s, Prolong<T> pro);
 // One full step on x.  z64 (float only, may be null): also the FP64 copy.
 template <typename T>
 int launch_small_symgs(const StencilLevel& L, const T* inv_diag, const T* r, T* x, double* z64,
-                       const double* ell_val, cudaStream_t s, Prolong<T> pro);
+                       const SmallEll* ell, cudaStream_t s, Prolong<T> pro);
 
 }  // namespace hb

@@ -46,13 +46,21 @@ bool small_level(const SparseMatrix& A, bool ell)
     return o && o->stencil_ok && hb::small_level_ok<T>(o->st, ell);
 }
 
-// A small level's zero-guess step and, where it has a coarse grid, the
-// restriction of its residual to rc, in one kernel.
-int small_zero_restrict(const SparseMatrix& A, const double* r, double* x, const double* ell_val, double* rc,
-                        cudaStream_t s, hb::Prolong<double> pro = {})
+hb::SmallEll small_ell(const SparseMatrix& A)
+{
+    const MGOpt* mo = mgopt(A);
+    return hb::SmallEll{A.ell_col_ind, A.ell_val, A.diag_idx, mo ? mo->inj_f : nullptr,
+                        mo ? A.Ac->localNumberOfRows : 0};
+}
+
+// A small level's zero-guess step (ell: on the ELL arrays) and, where rc is
+// given, the restriction of its residual to rc, in one kernel.
+int small_zero_restrict(const SparseMatrix& A, const double* r, double* x, bool ell, double* rc, cudaStream_t s,
+                        hb::Prolong<double> pro = {})
 {
     const LevelOpt* o = opt(A);
-    return hb::launch_small_zero<double>(o->st, o->diag, A.inv_diag, nullptr, const_cast<double*>(r), x, ell_val,
+    const hb::SmallEll e = small_ell(A);
+    return hb::launch_small_zero<double>(o->st, o->diag, A.inv_diag, nullptr, const_cast<double*>(r), x, ell ? &e : nullptr,
                                          rc ? mgopt(A)->inj_c : nullptr, rc, s, pro);
 }
 
@@ -69,7 +77,10 @@ int small_zero_restrict(const SparseMatrix& A, const double* r64, float* r, floa
 int symgs_ell(const SparseMatrix& A, const double* r, double* x, cudaStream_t s, hb::Prolong<double> pro = {})
 {
     if(small_level<double>(A, true))
-        return hb::launch_small_symgs<double>(opt(A)->st, A.inv_diag, r, x, nullptr, A.ell_val, s, pro);
+    {
+        const hb::SmallEll e = small_ell(A);
+        return hb::launch_small_symgs<double>(opt(A)->st, A.inv_diag, r, x, nullptr, &e, s, pro);
+    }
     return hb::launch_symgs(A.localNumberOfRows, A.nblocks, A.ublocks, A.sizes, A.offsets, A.ell_col_ind, A.ell_val,
                             A.inv_diag, r, x, s, pro);
 }
@@ -77,7 +88,7 @@ int symgs_ell(const SparseMatrix& A, const double* r, double* x, cudaStream_t s,
 int symgs_zero_ell(const SparseMatrix& A, const double* r, double* x, cudaStream_t s, hb::Prolong<double> pro = {})
 {
     const LevelOpt* o = opt(A);
-    if(small_level<double>(A, true)) return small_zero_restrict(A, r, x, A.ell_val, nullptr, s, pro);
+    if(small_level<double>(A, true)) return small_zero_restrict(A, r, x, true, nullptr, s, pro);
     return hb::launch_symgs_zero(A.localNumberOfRows, A.nblocks, A.ublocks, A.sizes, A.offsets, A.ell_col_ind,
                                  A.ell_val, A.diag_idx, o->diag, A.inv_diag, r, x, s, pro, zg_of(A));
 }
@@ -162,7 +173,7 @@ int mg64_ell(const SparseMatrix& A, const Vector& r, Vector& x, hb::Prolong<doub
     if(!A.mgData) return zero_guess(pro);
     const int pre = A.mgData->numberOfPresmootherSteps, post = A.mgData->numberOfPostsmootherSteps;
     if(pre == 1 && post > 0 && small_level<double>(A, true))
-        HB_RETURN_IF(small_zero_restrict(A, r.d_values, x.d_values, A.ell_val, A.mgData->rc->d_values, s));
+        HB_RETURN_IF(small_zero_restrict(A, r.d_values, x.d_values, true, A.mgData->rc->d_values, s));
     else
     {
         HB_RETURN_IF(zero_guess(post == 0 ? pro : hb::Prolong<double>{}));
@@ -275,7 +286,7 @@ int mg64_stencil(const SparseMatrix& A, const double* r, double* x, cudaStream_t
     // the coarsest level's zero-guess step is its last: it carries `pro`
     const hb::Prolong<double> pz = A.mgData ? hb::Prolong<double>{} : pro;
     if(small)
-        HB_RETURN_IF(small_zero_restrict(A, r, x, nullptr, A.mgData ? A.mgData->rc->d_values : nullptr, s, pz));
+        HB_RETURN_IF(small_zero_restrict(A, r, x, false, A.mgData ? A.mgData->rc->d_values : nullptr, s, pz));
     else if(stencil) HB_RETURN_IF(hb::launch64v_symgs_zero(o->st, o->diag, A.inv_diag, r, x, s, pz));
     else HB_RETURN_IF(symgs_zero_ell(A, r, x, s, pz));
     if(!A.mgData) return 0;

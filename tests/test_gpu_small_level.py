@@ -69,3 +69,84 @@ def test_full_step_with_any_values(dims, value):
                                        vp(P.device_ptr("diag")), vp(P.device_ptr("inv_diag")), vp(r), vp(y), s) == 0
         sync(P)
         assert torch.equal(x, y)
+
+
+def _vp(t):
+    return ctypes.c_void_p(t if isinstance(t, int) else t.data_ptr())
+
+
+def _launches(P, level, r, x, zero):
+    """One SymGS step of a level by the C ABI's launch-per-colour kernels on its present ELL arrays."""
+    sizes, offsets = P.field("sizes", level), P.field("offsets", level)
+    lay = (P.rows[level], 8, 6, sizes.ctypes.data_as(ctypes.c_void_p), offsets.ctypes.data_as(ctypes.c_void_p))
+    f = lambda *names: [_vp(P.device_ptr(n, level)) for n in names]  # noqa: E731
+    s = ctypes.c_void_p(P.stream_handle)
+    if zero:
+        rc = P.L.hpcgb200_symgs_zero(*lay, *f("ell_col", "ell_val", "diag_idx", "diag", "inv_diag"), _vp(r), _vp(x), s)
+    else:
+        rc = P.L.hpcgb200_symgs(*lay, *f("ell_col", "ell_val", "inv_diag"), _vp(r), _vp(x), s)
+    assert rc == 0
+
+
+def _change(P, what):
+    """Changes the level-0 ELL data of one row that has all its neighbours (and of one on a face)."""
+    m = P.rows[0]
+    col = dev_field(P, "ell_col", 0, np.int32).view(27, m)
+    val = dev_field(P, "ell_val", 0, np.float64).view(27, m)
+    inner = (col >= 0).all(0).nonzero().flatten()
+    row = int(inner[len(inner) // 3]) if what != "diagonal" else int(inner[-1])  # one that is restricted
+    face = int((col[26] < 0).nonzero().flatten()[0])
+    if what == "column":  # the neighbouring row of the same colour
+        col[4, row] += 1
+    elif what == "last column of a face row":  # a slot that its faces leave empty
+        col[26, face], val[26, face] = int(col[0, face]), -0.5
+    elif what == "diagonal":
+        val[int(dev_field(P, "diag_idx", 0, np.int32)[row]), row] = 30.0
+    elif what == "diagonals' slot":
+        dev_field(P, "diag_idx", 0, np.int32)[row] -= 1
+    elif what == "injection":
+        f = dev_field(P, "inj_f", 0, np.int32)
+        f[:2] = f[:2].flip(0).clone()
+    elif what == "value":
+        val[7, row] = -0.25
+    torch.cuda.synchronize()
+
+
+CHANGES = ["none", "column", "last column of a face row", "diagonal", "diagonals' slot", "value", "injection"]
+
+
+@pytest.mark.parametrize("dims", [(8, 8, 8), (16, 16, 16), (32, 24, 48)])
+@pytest.mark.parametrize("what", CHANGES)
+def test_cycle_on_changed_ell_arrays(dims, what):
+    """The FP64 operators are those of the ELL arrays as they are, on small levels too."""
+    with R.Problem(*dims, nlevels=2) as P:
+        n, s = P.rows, ctypes.c_void_p(P.stream_handle)
+        assert (dev_field(P, "inj_f", 0, np.int32).diff() == 1).all()  # what the one-cluster form counts on
+        g = torch.Generator(device="cuda").manual_seed(8)
+        r = torch.randn(n[0], dtype=torch.float64, device="cuda", generator=g)
+        x = torch.randn(n[0], dtype=torch.float64, device="cuda", generator=g)
+        _change(P, what)
+        y = x.clone()
+        torch.cuda.synchronize()
+        P.symgs(0, r.data_ptr(), x.data_ptr())
+        _launches(P, 0, r, y, False)
+        sync(P)
+        assert torch.equal(x, y)
+        P.symgs_zero(0, r.data_ptr(), x.data_ptr())
+        _launches(P, 0, r, y, True)
+        sync(P)
+        assert torch.equal(x, y)
+        # the V-cycle (src/ComputeMG.cpp:72-101)
+        rc, xc = (torch.zeros(n[1], dtype=torch.float64, device="cuda") for _ in range(2))
+        torch.cuda.synchronize()
+        f = lambda *names: [_vp(P.device_ptr(q)) for q in names]  # noqa: E731
+        assert P.L.hpcgb200_restrict_fused(n[1], *f("inj_f", "inj_c"), n[0], *f("ell_col", "ell_val"), _vp(r), _vp(y),
+                                           _vp(rc), s) == 0
+        _launches(P, 1, rc, xc, True)
+        sync(P)
+        inj = dev_field(P, "inj_f", 0, np.int32).long()
+        y[inj] += xc[dev_field(P, "inj_c", 0, np.int32).long()]
+        torch.cuda.synchronize()
+        _launches(P, 0, r, y, False)
+        sync(P)
+        assert np.array_equal(_mg(P, r, R.MODE_FP64), host(y))
