@@ -116,10 +116,12 @@ inline cudaError_t launch_pdl_smem(void (*kernel)(KArgs...), dim3 grid, dim3 blo
 }
 
 // Programmatic dependent launch for the learned smoother's kernels, inside
-// graphs too: each of them starts its dependents at entry, runs its prologue
-// (weights to shared memory, barriers, tensor memory) while the previous
-// kernel finishes, and waits (pdl_wait) before it touches that kernel's
-// output.  256^3 learned V-cycle 0.784 -> 0.773 ms, solve 0.178 -> 0.176 s
+// graphs too: each of them runs its prologue (weights to shared memory,
+// barriers, tensor memory) while the previous kernel finishes, starts its
+// dependents once it holds its tensor memory, and waits (pdl_wait) before it
+// touches the previous kernel's output.  A dependent allocates tensor memory
+// that it keeps until this kernel has ended: where it came first on an SM, this
+// kernel's own allocation would wait for it for ever.  256^3 learned V-cycle 0.784 -> 0.773 ms, solve 0.178 -> 0.176 s
 // (A/B on one box); HPCGB200_NET_PDL=0 turns it off.
 inline bool net_pdl_enabled()
 {
@@ -226,7 +228,9 @@ __device__ __forceinline__ void pdl_begin()
 }
 
 // The two halves of pdl_begin() for kernels with a prologue that does not
-// read the previous kernel's output (no-ops without the launch attribute).
+// read the previous kernel's output (no-ops without the launch attribute).  A
+// kernel starts its dependents only when it waits for nothing any more that
+// they may hold: tensor memory, above all.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -429,7 +429,6 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
              const __nv_bfloat16* __restrict__ act, PermMap pm, int* status)
 {
     extern __shared__ unsigned char smem_raw[];
-    pdl_launch_dependents();  // the next kernel may start its prologue
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* sA = smem;                                   // kStages x kStageBytes
     unsigned char* sW = smem + kStages * kStageBytes;           // weights
@@ -467,6 +466,7 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tholder;
+    pdl_launch_dependents();  // not before this CTA has its tensor memory
     pdl_wait();  // from here on the previous kernel's output is read
 
     if(warp == 0 && lane == 0)
@@ -708,7 +708,6 @@ __global__ void __launch_bounds__(k3Threads, 1)
                 PermMap pm, int* status)
 {
     extern __shared__ unsigned char smem_raw[];
-    pdl_launch_dependents();  // the next kernel may start its prologue
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* sA = smem;                                       // k3Stages x k3StageBytes
     unsigned char* sW = smem + k3Stages * k3StageBytes;             // + and - weight tiles
@@ -759,6 +758,7 @@ __global__ void __launch_bounds__(k3Threads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tholder;
+    pdl_launch_dependents();  // not before this CTA has its tensor memory
     pdl_wait();  // from here on the previous kernel's output is read
     constexpr uint32_t kBoxTx = (uint32_t)kCopyBytes * (kPair ? 2u : 1u);
 
@@ -1395,7 +1395,6 @@ __global__ void __launch_bounds__(k1Threads, k1CtasPerSm)
                 const __nv_bfloat16* __restrict__ act, int* status)
 {
     extern __shared__ unsigned char smem_raw[];
-    pdl_launch_dependents();  // the next kernel may start its prologue
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
     unsigned char* sA = smem;                     // k1Z planes of tap runs
     unsigned char* sW = sA + k1Z * k1PlaneBytes;  // weights
@@ -1421,6 +1420,7 @@ __global__ void __launch_bounds__(k1Threads, k1CtasPerSm)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tholder;
+    pdl_launch_dependents();  // not before this CTA has its tensor memory
     pdl_wait();  // from here on the previous kernel's output is read
 
     const long n = g.points();
