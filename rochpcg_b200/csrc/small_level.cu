@@ -145,9 +145,20 @@ __device__ __forceinline__ unsigned cluster_size()
     return r;
 }
 
-// The barrier between passes, in two halves; __syncthreads where one CTA has the whole level.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
+// The barrier between passes, in two halves; __syncthreads where one CTA has the
+// whole level.  The .aligned forms want the whole warp at one instruction, and
+// what stands before them is divergent (lanes without a row, copies to a
+// neighbour).
+__device__ __forceinline__ void cluster_arrive()
+{
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait()
+{
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
 
 // v into the same shared-memory cell of CTA `rank` of the cluster
 __device__ __forceinline__ void store_peer(double* cell, unsigned rank, double v)

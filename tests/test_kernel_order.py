@@ -33,3 +33,11 @@ def test_dependents_start_after_the_tensor_memory_is_held(kernel):
     assert all(i > held for i in starts)
     if kernel != "k_conv16_wgrad":
         assert len(starts) == 1 and starts[0] < body.index("pdl_wait(")
+
+
+def test_aligned_cluster_barriers_follow_a_converged_warp():
+    """barrier.cluster.*.aligned is undefined where the lanes of a warp arrive apart."""
+    text = _source("small_level.cu")
+    barriers = [m.start() for m in re.finditer(r'asm volatile\("barrier\.cluster\.\w+\.\w+\.aligned', text)]
+    assert len(barriers) == text.count("barrier.cluster") == 2
+    assert all(re.search(r"__syncwarp\(\);\s*$", text[:i]) for i in barriers)
