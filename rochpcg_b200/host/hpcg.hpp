@@ -240,7 +240,10 @@ int TestNorms(TestNormsData& testnorms_data);
 // the device: natural row order on the generated row-major arrays, so they
 // apply between GenerateCoarseProblem and OptimizeProblem (or later on a
 // hierarchy that keeps its generated arrays).  SpMV and SymGS results equal
-// the sequential C loops bit for bit.
+// the sequential C loops bit for bit.  ComputeSYMGS_ref, ComputeMG_ref and CG_ref
+// return when their result is there: HPCGB200_ERR_DEVICE_STATUS where a bounded
+// wait of a sweep ran out, x being undefined then (not while the stream is being
+// captured: the sweeps are launched front by front and wait for nothing).
 int ComputeSPMV_ref(const SparseMatrix& A, Vector& x, Vector& y);
 int ComputeSYMGS_ref(const SparseMatrix& A, const Vector& r, Vector& x);
 int ComputeMG_ref(const SparseMatrix& A, const Vector& r, Vector& x);

@@ -225,10 +225,6 @@ inline const hb::ZgGroups* zg_of(const SparseMatrix& A)
 }
 inline MGOpt* mgopt(const SparseMatrix& A) { return A.mgData ? static_cast<MGOpt*>(A.mgData->optimizationData) : nullptr; }
 
-// HPCGB200_ERR_DEVICE_STATUS if a reference sweep's wait ran out since the
-// last check (synchronises the stream), defined in reference.cpp.
-int reference_status();
-
 // Operators on raw FP32 level data (mixed V-cycle), defined in operators.cpp.
 // pro: where this level's final values are prolongated (the finer level's x),
 // fused into the level's last smoother passes; empty on level 0.

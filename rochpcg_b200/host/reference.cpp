@@ -57,24 +57,28 @@ int ComputeSPMV_ref(const SparseMatrix& A, Vector& x, Vector& y)
 
 namespace {
 
+bool capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    HB_HOST_CUDA(cudaStreamIsCapturing(s, &cs));
+    return cs != cudaStreamCaptureStatusNone;
+}
+
 // One symmetric sweep: the dataflow kernels (natural_flow.cu) with a
 // workspace kept beside the generated arrays, or one launch per front where a
-// plane has too many lines for them, the workspace cannot be had, or a
-// capture cannot allocate it.  104^3: 10.3 ms with the 1444 launches of
-// the fronts.  repeated: the previous sweep on this level had the
-// same matrix and r.
+// plane has too many lines for them, the workspace cannot be had, or the
+// stream is being captured (nobody could read the status of a replay's waits).
+// 104^3: 10.3 ms with the 1444 launches of the fronts.  repeated: the previous
+// sweep on this level had the same matrix and r.
 int symgs_ref(const SparseMatrix& A, const Vector& r, Vector& x, bool repeated)
 {
     const hb::NaturalLevel L = natural(A);
     cudaStream_t s = rt().stream;
-    if(hb::nat_flow_ok(L.nx, L.ny, L.nz))
+    if(hb::nat_flow_ok(L.nx, L.ny, L.nz) && !capturing(s))
     {
         if(!A.referenceData)
         {
-            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-            HB_CUDA(cudaStreamIsCapturing(s, &cs));
-            if(cs == cudaStreamCaptureStatusNone &&
-               cudaMalloc(&A.referenceData, hb::nat_flow_workspace_bytes(L.rows())) != cudaSuccess)
+            if(cudaMalloc(&A.referenceData, hb::nat_flow_workspace_bytes(L.rows())) != cudaSuccess)
             {
                 A.referenceData = nullptr;
                 cudaGetLastError();
@@ -87,10 +91,8 @@ int symgs_ref(const SparseMatrix& A, const Vector& r, Vector& x, bool repeated)
     return hb::launch_nat_symgs(L, r.d_values, x.d_values, s);
 }
 
-}  // namespace
-
-namespace hpcg_b200 {
-
+// HPCGB200_ERR_DEVICE_STATUS if a reference sweep's wait ran out since the
+// last check (synchronises the stream).
 int reference_status()
 {
     int h = 0;
@@ -101,12 +103,21 @@ int reference_status()
     return hb::record_error(HPCGB200_ERR_DEVICE_STATUS, "reference Gauss-Seidel: a bounded device wait timed out");
 }
 
-}  // namespace hpcg_b200
+// The end of every public operator that runs sweeps, whatever its rc: it takes
+// the status with it, so that none is left to another call.
+int with_status(int rc)
+{
+    if(capturing(rt().stream)) return rc;
+    const int status = reference_status();
+    return rc ? rc : status;
+}
+
+}  // namespace
 
 // src/ComputeSYMGS_ref.cpp:51-104
 int ComputeSYMGS_ref(const SparseMatrix& A, const Vector& r, Vector& x)
 {
-    return guarded([&] { return symgs_ref(A, r, x, false); });
+    return guarded([&] { return with_status(symgs_ref(A, r, x, false)); });
 }
 
 // src/ComputeRestriction_ref.cpp:41-56
@@ -131,8 +142,10 @@ int ComputeProlongation_ref(const SparseMatrix& Af, Vector& xf)
     });
 }
 
-// src/ComputeMG_ref.cpp:37-62
-int ComputeMG_ref(const SparseMatrix& A, const Vector& r, Vector& x)
+namespace {
+
+// src/ComputeMG_ref.cpp:37-62, without the look at the status
+int mg_ref(const SparseMatrix& A, const Vector& r, Vector& x)
 {
     HB_RETURN_IF(guarded([&] {
         CudaZeroVector(x);
@@ -151,12 +164,19 @@ int ComputeMG_ref(const SparseMatrix& A, const Vector& r, Vector& x)
         if(ierr) return ierr;
         HB_RETURN_IF(ComputeSPMV_ref(A, x, *A.mgData->Axf));
         HB_RETURN_IF(ComputeRestriction_ref(A, r));
-        HB_RETURN_IF(ComputeMG_ref(*A.Ac, *A.mgData->rc, *A.mgData->xc));
+        HB_RETURN_IF(mg_ref(*A.Ac, *A.mgData->rc, *A.mgData->xc));
         HB_RETURN_IF(ComputeProlongation_ref(A, x));
         for(int i = 0; i < A.mgData->numberOfPostsmootherSteps; ++i) ierr += smooth();
         return ierr;
     }
-    return ComputeSYMGS_ref(A, r, x);
+    return guarded([&] { return symgs_ref(A, r, x, false); });
+}
+
+}  // namespace
+
+int ComputeMG_ref(const SparseMatrix& A, const Vector& r, Vector& x)
+{
+    return guarded([&] { return with_status(mg_ref(A, r, x)); });
 }
 
 // src/ComputeDotProduct_ref.cpp:46-80 (one rank: no allreduce)
@@ -181,10 +201,11 @@ int ComputeWAXPBY_ref(local_int_t n, double alpha, const Vector& x, double beta,
 
 // src/CG_ref.cpp:60-160: the recurrence, operator order and timing slots of
 // the reference CG (times[1] dots, [2] WAXPBY, [3] SpMV, [5] MG, [0] total;
-// every phase is synchronised so the split is meaningful).
-int CG_ref(const SparseMatrix& A, CGData& data, const Vector& b, Vector& x, const int max_iter,
-           const double tolerance, int& niters, double& normr, double& normr0, double* times, bool doPreconditioning,
-           bool verbose)
+// every phase is synchronised so the split is meaningful), without the look at
+// the sweeps' status.
+static int cg_ref(const SparseMatrix& A, CGData& data, const Vector& b, Vector& x, const int max_iter,
+                  const double tolerance, int& niters, double& normr, double& normr0, double* times,
+                  bool doPreconditioning, bool verbose)
 {
     try
     {
@@ -224,7 +245,7 @@ int CG_ref(const SparseMatrix& A, CGData& data, const Vector& b, Vector& x, cons
         for(int k = 1; k <= max_iter && normr / normr0 > tolerance; k++)
         {
             tick();
-            if(doPreconditioning) HB_RETURN_IF(ComputeMG_ref(A, r, z));
+            if(doPreconditioning) HB_RETURN_IF(mg_ref(A, r, z));
             else HB_RETURN_IF(ComputeWAXPBY_ref(nrow, 1.0, r, 0.0, r, z));
             tock(t5);
             if(k == 1)
@@ -273,12 +294,22 @@ int CG_ref(const SparseMatrix& A, CGData& data, const Vector& b, Vector& x, cons
             times[5] += t5;
             times[0] += now() - t_begin;
         }
-        return reference_status();
+        return 0;
     }
     catch(const Error& e)
     {
         return report(e);
     }
+}
+
+int CG_ref(const SparseMatrix& A, CGData& data, const Vector& b, Vector& x, const int max_iter,
+           const double tolerance, int& niters, double& normr, double& normr0, double* times, bool doPreconditioning,
+           bool verbose)
+{
+    return guarded([&] {
+        return with_status(cg_ref(A, data, b, x, max_iter, tolerance, niters, normr, normr0, times, doPreconditioning,
+                                  verbose));
+    });
 }
 
 // src/CheckProblem.cpp:79-150, counting mismatching rows instead of asserting.
