@@ -417,7 +417,8 @@ __global__ void __launch_bounds__(kBS) k_nat_check_rows(NaturalLevel L, double* 
 }
 
 // Natural order [iz][iy][ix] <-> [iz][(ix + 2 iy) mod nx][iy], a 32 x 32 tile
-// of a plane through shared memory per block.
+// of a plane through shared memory per block.  The planes are the grid's x: there
+// may be more than 65535 of them.
 constexpr int kTile = 32;
 
 template <bool kTo>
@@ -426,8 +427,8 @@ __global__ void __launch_bounds__(kBS) k_nat_skew(int nx, int ny, const double* 
 {
     __shared__ double tile[kTile][kTile + 1];
     if(!kTo && *other) return;
-    const int x0 = blockIdx.x * kTile, y0 = blockIdx.y * kTile;
-    const size_t plane = (size_t)blockIdx.z * nx * ny;
+    const int x0 = blockIdx.y * kTile, y0 = blockIdx.z * kTile;
+    const size_t plane = (size_t)blockIdx.x * nx * ny;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     auto natural = [&](auto f) {
         for(int j = warp; j < kTile; j += kBS / 32)
@@ -537,7 +538,7 @@ int launch_nat_symgs_flow(const NaturalLevel& L, const double* r, double* x, voi
 {
     const size_t m = (size_t)L.rows();
     const Workspace w = carve(workspace, m);
-    const dim3 tiles((unsigned)((L.nx + kTile - 1) / kTile), (unsigned)((L.ny + kTile - 1) / kTile), (unsigned)L.nz);
+    const dim3 tiles((unsigned)L.nz, (unsigned)((L.nx + kTile - 1) / kTile), (unsigned)((L.ny + kTile - 1) / kTile));
 
     HB_CUDA(cudaMemsetAsync(w.x1, 0xff, 2 * m * sizeof(double), s));
     if(!prepared)

@@ -69,6 +69,12 @@ def test_reference_cycle_is_the_front_by_front_one(dims):
             _compare(P, _normal(P, seed))
 
 
+def test_more_planes_than_a_grid_has_in_z():
+    """Launch dimensions y and z end at 65535."""
+    with R.Problem(4, 4, 65544, nlevels=1, keep_generated=True) as P:
+        _compare(P, _normal(P, 5))
+
+
 @pytest.mark.parametrize("level", [0, 1])
 @pytest.mark.parametrize("slot", [0, 26])
 def test_changed_matrix_takes_the_general_sweep(level, slot):
