@@ -277,12 +277,14 @@ bool stencil_vec_level(const SparseMatrix& A)
 
 // ComputeMG's recursion (1 zero-guess pre-smoothing step, fused restriction,
 // coarse solve, prolongation, 1 post-smoothing step) per level on the
-// implicit-stencil kernels or, where the level is not the verified stencil,
-// the ELL ones.
+// implicit-stencil kernels or, where the level is not the verified stencil
+// or has too many planes for the one-row ones, the ELL ones.
 int mg64_stencil(const SparseMatrix& A, const double* r, double* x, cudaStream_t s, hb::Prolong<double> pro)
 {
     const LevelOpt* o = opt(A);
-    const bool stencil = o && o->stencil_ok, vec = stencil_vec_level(A), small = small_level<double>(A, false);
+    const bool vec = stencil_vec_level(A), small = small_level<double>(A, false);
+    // the one-row kernels have a colour's planes on their grid's z axis
+    const bool stencil = vec || (o && o->stencil_ok && o->st.nz <= 2 * 65535);
     // the coarsest level's zero-guess step is its last: it carries `pro`
     const hb::Prolong<double> pz = A.mgData ? hb::Prolong<double>{} : pro;
     if(small)

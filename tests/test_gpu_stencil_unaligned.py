@@ -11,7 +11,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dims,nlevels", [((52, 52, 52), 1), ((100, 84, 68), 2), ((104, 104, 104), 2), ((66, 62, 34), 1),
-                                          ((51, 43, 71), 1), ((130, 34, 46), 1), ((129, 65, 33), 1)])
+                                          ((51, 43, 71), 1), ((130, 34, 46), 1), ((129, 65, 33), 1),
+                                          # as many planes as a launch's z axis holds, and more
+                                          ((4, 4, 131070), 1), ((4, 4, 131080), 1)])
 def test_cycle_is_the_ell_one(dims, nlevels):
     with R.Problem(*dims, nlevels=nlevels) as P:
         assert P.stencil_ok(0)
