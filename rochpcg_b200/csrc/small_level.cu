@@ -17,10 +17,9 @@
 // one-launch kernels: the same sums, bit for bit.
 //
 // A zero-guess step in a graph, one cluster against 15 launches: 16^3 FP32 18.6
-// against 26.8 us, FP64 20.6 against 32.8, ELL arrays 20.5 against 42.5; 32^3 20.6
-// / 30.8, 22.6 / 36.9, 30.7 / 45.1 (the check of 27 slots a row is 8 us of it).
-// The whole V-cycle called through the operator API: 16^3 FP64 446 -> 137 us,
-// 104^3 mixed 466 -> 334 us.
+// against 26.8 us, FP64 20.6 against 32.8, ELL arrays 20.5 against 45.1; 32^3 20.6
+// / 30.8, 22.6 / 36.9, 26.6 / 45.2.  The whole V-cycle called through the operator
+// API: 16^3 FP64 446 -> 134 us, 104^3 mixed 466 -> 334 us.
 #include <algorithm>
 #include <type_traits>
 
@@ -34,7 +33,7 @@ constexpr int kMaxCtas = 16;
 // A thread has one row of each colour, so a level fits where a CTA's share of a
 // pass does: 640 threads leave 96 registers (48 x 24 x 40 with 576 gains, 28.3
 // against 31.3 us; two rows a thread at 40^3 lost, 40.4 against 32.8 us), the
-// ELL form needs 112 and always takes its 512, which read the arrays.
+// ELL form needs 112.
 constexpr int kMaxThreads = 640, kMaxThreadsEll = 512;
 constexpr int kSmallSmem = 220 * 1024;
 constexpr int kOneCta = 2048;    // rows of a level up to which one CTA takes it: no cluster barrier (8^3 20.5 -> 14.5 us)
@@ -103,7 +102,6 @@ struct SmallArgs
 struct EllArgs
 {
     SmallEll m;
-    int rows;              // rows of a pass and CTA at most, a multiple of 32
     int dcol[8][27];       // by stencil point: its column in a row of a colour, from the row's brick position
     signed char slot[8][27];  // and its slot
 };
@@ -175,16 +173,6 @@ __device__ __forceinline__ void store_peer(float* cell, unsigned rank, float v)
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(p), "f"(v) : "memory");
 }
 
-// the int cell of CTA `rank` of the cluster
-__device__ __forceinline__ int load_peer(const int* cell, unsigned rank)
-{
-    unsigned a = (unsigned)__cvta_generic_to_shared(cell), p;
-    int v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(p) : "r"(a), "r"(rank));
-    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(p) : "memory");
-    return v;
-}
-
 __device__ __forceinline__ float mul_once(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_once(double a, double b) { return __dmul_rn(a, b); }
 
@@ -228,6 +216,72 @@ __device__ double any_row(const SmallArgs<double>& a, const SmallEll& e, int row
     return sum * a.inv_diag[row];
 }
 
+// t / n for 0 <= t < 2^20
+__device__ __forceinline__ int quotient(int t, int n) { return __float2int_rd(((float)t + 0.5f) * __frcp_rn((float)n)); }
+
+// Not 0 where row t of colour v is not the stencil's in the ELL arrays, its
+// diagonal slot or (zero guess) its diagonal, or is injected elsewhere.
+template <bool kZero>
+__device__ __forceinline__ unsigned row_differs(const SmallArgs<double>& a, const EllArgs& ell, int v, int t)
+{
+    const int cls = c_order.cls[v], px = (cls >> 2) & 1, py = (cls >> 1) & 1, pz = cls & 1;
+    const int bx = (a.nx - px + 1) / 2, by = (a.ny - py + 1) / 2;
+    const int q = quotient(t, bx), kx = t - q * bx, kz = quotient(q, by), ky = q - kz * by;
+    const int g = a.off[v] + t;
+    const int ix = 2 * kx + px, iy = 2 * ky + py, iz = 2 * kz + pz;
+    const unsigned* face = c_order.gone[v];
+    const unsigned gone = (ix == 0 ? face[0] : 0u) | (ix == a.nx - 1 ? face[1] : 0u) | (iy == 0 ? face[2] : 0u) |
+                          (iy == a.ny - 1 ? face[3] : 0u) | (iz == 0 ? face[4] : 0u) |
+                          (iz == a.nz - 1 ? face[5] : 0u);
+    // the row's position in the neighbours' bricks: index bit 0 dx odd, bit 1 dy odd
+    int at[4];
+#pragma unroll
+    for(int k = 0; k < 4; ++k)
+        at[k] = (kz * ((a.ny + 1 - (py ^ (k >> 1))) / 2) + ky) * ((a.nx + 1 - (px ^ (k & 1))) / 2) + kx;
+    const double diag = kZero ? __ldg(a.diag + g) : 0.0;
+    unsigned other = 0;
+    // slots are packed: those the faces remove leave the row's last ones empty
+#pragma unroll
+    for(int n = 0; n < 27; ++n)
+    {
+        const int j = ell.slot[v][n], missing = __popc(gone & ((1u << j) - 1u));
+        const bool off = gone >> j & 1u;
+        const int at_e = (off ? 26 - missing : j - missing) * a.m + g;
+        const unsigned c = (unsigned)__ldg(ell.m.col + at_e);
+        const unsigned want = (unsigned)(at[(n % 3 != 1) + 2 * (n / 3 % 3 != 1)] + ell.dcol[v][n]);
+        unsigned differs = c ^ want;
+        if(n != 13 || kZero) differs |= __ldg(ell.m.val + at_e) == (n == 13 ? diag : -1.0) ? 0u : 1u;
+        other |= off ? (unsigned)(c < (unsigned)a.m) : differs;
+    }
+    if constexpr(kZero)
+    {
+        const int dp = c_order.dp[v];
+        other |= (unsigned)(__ldg(ell.m.diag_idx + g) ^ (dp - __popc(gone & ((1u << dp) - 1u))));
+        if(a.rc && v == 7) other |= (unsigned)(__ldg(ell.m.inj_f + t) ^ g);
+    }
+    return other;
+}
+
+// Sets *ell.m.changed where some row differs.  A kernel of its own: a level's
+// arrays are up to 21 MB, which the cluster's 16 SMs alone take 12 us to read
+// (64 x 32 x 32 zero-guess step 45.1 us with the check in its prologue, 32.7 so;
+// 16^3 20.5 either way).
+template <bool kZero>
+__global__ void __launch_bounds__(kBS)
+    k_small_check(const __grid_constant__ SmallArgs<double> a, const __grid_constant__ EllArgs ell)
+{
+    pdl_launch_dependents();
+    const int g = blockIdx.x * kBS + threadIdx.x;
+    unsigned other = 0;
+    if(g < a.m)
+    {
+        int v = 0;
+        while(v < 7 && g >= a.off[v + 1]) ++v;
+        other = row_differs<kZero>(a, ell, v, g - a.off[v]);
+    }
+    if(__syncthreads_or((int)other) && threadIdx.x == 0) atomicExch(ell.m.changed, 1);
+}
+
 // The dynamic shared memory: the x bricks, then per colour and thread the
 // row's r, 1/a_ii and (zero guess) a_ii, and its cell.
 template <typename T, bool kZero>
@@ -239,10 +293,10 @@ constexpr int kNone = -1, kToBelow = 1 << 30, kToAbove = 1 << 29, kCellMask = kT
 // kZero: the zero-guess step (forward pass: slots before the diagonal,
 // backward: a_ii x_i and the slots after it) and, with rc given, the
 // restriction of its residual; else the full step.  kEll: the step is that of
-// the ELL arrays as they are now -- they are read once, before the first pass.
-// Where every column, value and diagonal slot of the cluster's rows is the
-// stencil's, the passes are the implicit ones (sum + x is fma(1, x, sum)); else
-// the cluster runs them on the arrays, with x in global memory.  A thread has at most one row of each colour; what a pass needs of it
+// the ELL arrays as they are now -- k_small_check has read them just before.
+// Where every column, value and diagonal slot is the stencil's, the passes are
+// the implicit ones (sum + x is fma(1, x, sum)); else the cluster runs them on
+// the arrays, with x in global memory.  A thread has at most one row of each colour; what a pass needs of it
 // besides its neighbours' x is fetched between the barrier's arrival and its
 // wait.
 template <typename T, bool kZero, bool kEll>
@@ -260,7 +314,6 @@ __global__ void __launch_bounds__(kEll ? kMaxThreadsEll : kMaxThreads, 1)
     __shared__ __align__(16) int s_tab[8][28];  // per colour: cell offset of each slot but the diagonal's, in order
     __shared__ int s_row0[8];                   // per colour: the CTA's first row
     __shared__ int s_dp[8];                     // per colour: the diagonal's slot
-    __shared__ int s_other;                     // kEll: some row of this CTA is not the stencil's
     const unsigned rank = cluster_rank(), size = cluster_size();
     const int p0 = (int)(rank * (unsigned)a.pairs / size), p1 = (int)((rank + 1) * (unsigned)a.pairs / size);
     const int np = p1 - p0;
@@ -271,11 +324,8 @@ __global__ void __launch_bounds__(kEll ? kMaxThreadsEll : kMaxThreads, 1)
     auto cell_of = [&](int hx, int hy, int hz) {
         return (((hx & 1) << 2) | ((hy & 1) << 1) | (hz & 1)) * a.brick + (hz >> 1) * sxy + (hy >> 1) * a.sx + (hx >> 1);
     };
-    // t / n for 0 <= t < 2^20
-    auto quotient = [](int t, int n) { return __float2int_rd(((float)t + 0.5f) * __frcp_rn((float)n)); };
 
     // this thread's row of every colour
-    unsigned other = 0;  // kEll: bits in which rows differ from the stencil's
 #pragma unroll
     for(int v = 0; v < 8; ++v)
     {
@@ -306,52 +356,6 @@ __global__ void __launch_bounds__(kEll ? kMaxThreadsEll : kMaxThreads, 1)
         else r = __ldg(a.r + g);
         s_r[v * nt] = r;
     }
-    if constexpr(kEll)
-    {
-        // All threads of a full block, a row of some colour each (by the rows' own
-        // threads, unrolled over the colours: 16^3 V-cycle 133 -> 205 us).
-#pragma unroll 1
-        for(int e = tid; e < 8 * ell.rows; e += nt)
-        {
-            const int v = e / ell.rows, t = e - v * ell.rows;
-            const int cls = c_order.cls[v], px = (cls >> 2) & 1, py = (cls >> 1) & 1, pz = cls & 1;
-            const int bx = (a.nx - px + 1) / 2, by = (a.ny - py + 1) / 2, bz = (a.nz - pz + 1) / 2;
-            if(t >= (min(p1, bz) - p0) * by * bx) continue;
-            const int q = quotient(t, bx), kx = t - q * bx, kp = quotient(q, by), ky = q - kp * by, kz = p0 + kp;
-            const int g = a.off[v] + p0 * by * bx + t;
-            const int ix = 2 * kx + px, iy = 2 * ky + py, iz = 2 * kz + pz;
-            const unsigned* face = c_order.gone[v];
-            const unsigned gone = (ix == 0 ? face[0] : 0u) | (ix == a.nx - 1 ? face[1] : 0u) |
-                                  (iy == 0 ? face[2] : 0u) | (iy == a.ny - 1 ? face[3] : 0u) |
-                                  (iz == 0 ? face[4] : 0u) | (iz == a.nz - 1 ? face[5] : 0u);
-            // the row's position in the neighbours' bricks: index bit 0 dx odd, bit 1 dy odd
-            int at[4];
-#pragma unroll
-            for(int k = 0; k < 4; ++k)
-                at[k] = (kz * ((a.ny + 1 - (py ^ (k >> 1))) / 2) + ky) * ((a.nx + 1 - (px ^ (k & 1))) / 2) + kx;
-            const double diag = kZero ? __ldg(a.diag + g) : 0.0;
-            // slots are packed: those the faces remove leave the row's last ones empty
-#pragma unroll
-            for(int n = 0; n < 27; ++n)
-            {
-                const int j = ell.slot[v][n], missing = __popc(gone & ((1u << j) - 1u));
-                const bool off = gone >> j & 1u;
-                const int at_e = (off ? 26 - missing : j - missing) * a.m + g;
-                const unsigned c = (unsigned)__ldg(ell.m.col + at_e);
-                const unsigned want = (unsigned)(at[(n % 3 != 1) + 2 * (n / 3 % 3 != 1)] + ell.dcol[v][n]);
-                unsigned differs = c ^ want;
-                if(n != 13 || kZero)
-                    differs |= __ldg(ell.m.val + at_e) == (n == 13 ? diag : -1.0) ? 0u : 1u;
-                other |= off ? (unsigned)(c < (unsigned)a.m) : differs;
-            }
-            if constexpr(kZero)
-            {
-                const int dp = c_order.dp[v];
-                other |= (unsigned)(__ldg(ell.m.diag_idx + g) ^ (dp - __popc(gone & ((1u << dp) - 1u))));
-                if(a.rc && v == 7) other |= (unsigned)(__ldg(ell.m.inj_f + (g - a.off[7])) ^ g);
-            }
-        }
-    }
     for(int e = tid; e < 8 * a.brick; e += nt) xs[e] = T(-0.0);
     for(int e = tid; e < 8 * 28; e += nt)
     {
@@ -362,12 +366,7 @@ __global__ void __launch_bounds__(kEll ? kMaxThreadsEll : kMaxThreads, 1)
                 cell_of(hx + c_order.dx[v][j], hy + c_order.dy[v][j], hz + c_order.dz[v][j]) - cell_of(hx, hy, hz);
         else if(j == 27) s_tab[v][26] = s_tab[v][27] = 0;
     }
-    if constexpr(kEll)
-    {
-        const int any = __syncthreads_or((int)other);
-        if(tid == 0) s_other = any;
-    }
-    else __syncthreads();
+    __syncthreads();
     if constexpr(!kZero)
     {
         for(int v = 0; v < 8; ++v)
@@ -420,13 +419,8 @@ __global__ void __launch_bounds__(kEll ? kMaxThreadsEll : kMaxThreads, 1)
     wait();
     if constexpr(kEll)
     {
-        int any = s_other;
-        if(size > 1)
-        {
-            const int lane = tid & 31;
-            any = __any_sync(0xffffffffu, lane < (int)size ? load_peer(&s_other, (unsigned)lane) : 0);
-        }
-        if(any)
+        pdl_wait();
+        if(__ldcg(ell.m.changed))
         {
 #pragma unroll 1
             for(int i = 0; i < 15; ++i)
@@ -442,12 +436,16 @@ __global__ void __launch_bounds__(kEll ? kMaxThreadsEll : kMaxThreads, 1)
                 arrive();
                 wait();
             }
-            if(!kZero || !a.rc) return;
-            for(int ic = (int)rank * nt + tid; ic < ell.m.nc; ic += (int)size * nt)
+            if(rank == 0 && tid == 0) *ell.m.changed = 0;  // everyone has read it
+            if constexpr(kZero)
             {
-                const int row = ell.m.inj_f[ic], m = a.m;
-                a.rc[a.inj_c[ic]] = ell_row_sum(m, row, ell.m.col, ell.m.val, L2Reads{a.x}, a.r[row], -1.0, 0, kWidth,
-                                                [m](int col) { return col >= 0 && col < m; });
+                const int nc = a.rc ? ell.m.nc : 0, m = a.m;
+                for(int ic = (int)rank * nt + tid; ic < nc; ic += (int)size * nt)
+                {
+                    const int row = ell.m.inj_f[ic];
+                    a.rc[a.inj_c[ic]] = ell_row_sum(m, row, ell.m.col, ell.m.val, L2Reads{a.x}, a.r[row], -1.0, 0,
+                                                    kWidth, [m](int col) { return col >= 0 && col < m; });
+                }
             }
             return;
         }
@@ -539,12 +537,11 @@ int max_ctas()
 // Cluster shape of a level.
 struct Shape
 {
-    int ctas, per;      // z-plane pairs of a CTA at most
-    int rows, threads;  // rows of a pass and CTA at most, in whole warps
+    int ctas, threads, per;  // per: z-plane pairs of a CTA at most
     size_t smem;
 };
 
-template <typename T, bool kEll>
+template <typename T>
 Shape shape_of(const StencilLevel& L)
 {
     Shape s{};
@@ -555,8 +552,7 @@ Shape shape_of(const StencilLevel& L)
     while(s.ctas > pairs) s.ctas /= 2;
     s.per = (pairs + s.ctas - 1) / s.ctas;
     const int rows = ((L.nx + 1) / 2) * ((L.ny + 1) / 2) * s.per;
-    s.rows = (rows + 31) / 32 * 32;
-    s.threads = kEll ? kMaxThreadsEll : s.rows;
+    s.threads = (rows + 31) / 32 * 32;
     s.smem = sizeof(T) * 8 * (size_t)((L.nx + 3) / 2) * ((L.ny + 3) / 2) * (s.per + 1) +
              bytes_per_thread<T, true> * (size_t)s.threads;
     return s;
@@ -578,20 +574,21 @@ SmallArgs<T> args_of(const StencilLevel& L)
 }
 
 template <typename T, bool kZero, bool kEll>
-int launch_shape(const StencilLevel& L, SmallArgs<T> a, std::conditional_t<kEll, EllArgs, NoEll> ell,
+int launch_shape(const StencilLevel& L, SmallArgs<T> a, const std::conditional_t<kEll, EllArgs, NoEll>& ell,
                  cudaStream_t s)
 {
-    const Shape sh = shape_of<T, kEll>(L);
+    const Shape sh = shape_of<T>(L);
     a.brick = a.sx * a.sy * (sh.per + 1);
-    if constexpr(kEll) ell.rows = sh.rows;
     const auto kernel = k_small_symgs<T, kZero, kEll>;
     HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem));
     HB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)sh.ctas;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)sh.ctas);
     cfg.blockDim = dim3((unsigned)sh.threads);
@@ -599,6 +596,12 @@ int launch_shape(const StencilLevel& L, SmallArgs<T> a, std::conditional_t<kEll,
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    if constexpr(kEll)
+    {
+        k_small_check<kZero><<<(a.m + kBS - 1) / kBS, kBS, 0, s>>>(a, ell);
+        HB_LAUNCHED();
+        cfg.numAttrs = 2;  // the passes' kernel sets itself up meanwhile
+    }
     HB_CUDA(cudaLaunchKernelEx(&cfg, kernel, a, ell));
     return 0;
 }
@@ -625,8 +628,8 @@ bool small_level_ok(const StencilLevel& L, bool ell)
     if(L.ncolors != 8 || L.m > kMostRows) return false;
     for(int p = 0; p < 8; ++p)
         if(L.color_of_par[p] != colour_of(p)) return false;
-    const Shape s = ell ? shape_of<T, true>(L) : shape_of<T, false>(L);
-    return s.rows <= (ell ? kMaxThreadsEll : kMaxThreads) && s.smem <= kSmallSmem;
+    const Shape s = shape_of<T>(L);
+    return s.threads <= (ell ? kMaxThreadsEll : kMaxThreads) && s.smem <= kSmallSmem;
 }
 
 template <typename T>

@@ -24,6 +24,7 @@ struct SmallEll
     const int* diag_idx;
     const int* inj_f;  // with nc: the restriction's
     int nc;
+    int* changed;      // device word, 0 between steps
 };
 
 // One zero-guess step: x from r; r64 (float only, may be null): r comes in

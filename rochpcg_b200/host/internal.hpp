@@ -173,6 +173,7 @@ struct LevelOpt
     float* inv_diag32 = nullptr;
     int* pass_status = nullptr;        // set (3) by a TMA-staged colour pass whose copies timed out (device word;
                                        // never cleared: every later solve on the problem reports it)
+    int* ell_changed = nullptr;        // device word of the small-level SymGS's check of the ELL arrays
 
     // level-0 solver state
     hb::CGState* cg_state = nullptr;

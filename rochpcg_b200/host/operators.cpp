@@ -50,7 +50,7 @@ hb::SmallEll small_ell(const SparseMatrix& A)
 {
     const MGOpt* mo = mgopt(A);
     return hb::SmallEll{A.ell_col_ind, A.ell_val, A.diag_idx, mo ? mo->inj_f : nullptr,
-                        mo ? A.Ac->localNumberOfRows : 0};
+                        mo ? A.Ac->localNumberOfRows : 0, opt(A)->ell_changed};
 }
 
 // A small level's zero-guess step (ell: on the ELL arrays) and, where rc is

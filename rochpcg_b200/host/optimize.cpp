@@ -100,6 +100,8 @@ static void optimize_level(SparseMatrix& A)
         o->pass_status = dalloc<int>(1);
         HB_HOST_CUDA(cudaMemsetAsync(o->pass_status, 0, sizeof(int), s));
         o->st.status = o->pass_status;
+        o->ell_changed = dalloc<int>(1);
+        HB_HOST_CUDA(cudaMemsetAsync(o->ell_changed, 0, sizeof(int), s));
         o->diag32 = dalloc<float>(m);
         o->inv_diag32 = dalloc<float>(m);
         check(hb::launch_diag32(m, o->diag, o->diag32, o->inv_diag32, s));
