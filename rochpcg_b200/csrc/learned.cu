@@ -283,7 +283,7 @@ __host__ __device__ constexpr int weight_slot(int t) { return ((t / 3) % 3) * 9 
 //               brick (21 for kTZ = 4) into one of two accumulators of
 //               kTZ x 48 columns;
 //   warps 2-9   epilogue: tcgen05.ld of the finished accumulator, the dx
-//               combination, ReLU / mask / permuted scatter, global stores
+//               combination, ReLU / mask, global stores
 //               (eight warps instead of four: a training batch, whose masked
 //               passes read the activations too, 371 -> 361 us).
 // Two samples of 128^3 took 96 us; with a sixth of the box rows loaded 94, a
@@ -426,7 +426,7 @@ __device__ __forceinline__ bool role_wait(uint64_t* mbar, uint32_t parity, volat
 template <int kOut>
 __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
     k_conv16(const __grid_constant__ CUtensorMap in_map, ConvGrid g, const __nv_bfloat16* __restrict__ wB, void* out,
-             const __nv_bfloat16* __restrict__ act, PermMap pm, int* status)
+             const __nv_bfloat16* __restrict__ act, int* status)
 {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -638,15 +638,9 @@ __global__ void __launch_bounds__(kConvThreads, HB_CONV_CTAS)
                     for(int c = 0; c < 4; ++c)
                         dst[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
                 }
-                else if constexpr(kOut == kOutF32C0)
-                {
-                    reinterpret_cast<float*>(out)[p] = v[0];
-                }
                 else
                 {
-                    float* xo = reinterpret_cast<float*>(out) + perm_row(pm, z, y, x);
-                    if constexpr(kOut == kOutPermSet) *xo = v[0];
-                    else *xo += v[0];
+                    reinterpret_cast<float*>(out)[p] = v[0];
                 }
             };
             // the second plane's columns on their way while the first is finished
@@ -1163,52 +1157,6 @@ __device__ __forceinline__ void store_embed(__nv_bfloat16* a, long p, float r0)
     store_point(a + p * kNetCh, pack_bf16x8(v), make_uint4(0, 0, 0, 0));
 }
 
-// Channel 0 = r (x == nullptr) or the residual r - A x of the 27-point
-// stencil (diagonal diag32, off-diagonals -1), read from colour-permuted
-// level vectors at natural point p.
-__global__ void k_embed_level(PermMap pm, int nz, int ny, int nx, const float* __restrict__ r,
-                              const float* __restrict__ x, const float* __restrict__ diag32,
-                              __nv_bfloat16* __restrict__ a, int pair)
-{
-    const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if(p >= (long)nz * ny * nx) return;
-    const int z = (int)(p / ((long)ny * nx));
-    const long rem = p - (long)z * ny * nx;
-    const int y = (int)(rem / nx), xx = (int)(rem - (long)y * nx);
-    const int row = perm_row(pm, z, y, xx);
-    float v = r[row];
-    if(x)
-    {
-        float off = 0.f;
-#pragma unroll
-        for(int t = 0; t < 27; ++t)
-        {
-            const int z2 = z + t / 9 - 1, y2 = y + (t / 3) % 3 - 1, x2 = xx + t % 3 - 1;
-            if(t != 13 && z2 >= 0 && z2 < nz && y2 >= 0 && y2 < ny && x2 >= 0 && x2 < nx)
-                off += x[perm_row(pm, z2, y2, x2)];
-        }
-        v = v - (diag32[row] * x[row] - off);
-    }
-    store_embed(a, p, v);
-    if(pair) store_embed(a, p + (long)nz * ny * nx, -v);  // second sample: -v (odd evaluation)
-}
-
-// x[row(p)] = (or +=) (y[p] - y[p + n]) / 2: the odd part of the network.
-template <bool kAdd>
-__global__ void k_odd_combine(PermMap pm, int nz, int ny, int nx, const float* __restrict__ y, float* __restrict__ x)
-{
-    const long n = (long)nz * ny * nx;
-    const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if(p >= n) return;
-    const int z = (int)(p / ((long)ny * nx));
-    const long rem = p - (long)z * ny * nx;
-    const int yy = (int)(rem / nx), xx = (int)(rem - (long)yy * nx);
-    const float v = 0.5f * (y[p] - y[p + n]);
-    float* o = x + perm_row(pm, z, yy, xx);
-    if(kAdd) *o += v;
-    else *o = v;
-}
-
 // Natural <-> colour-permuted copies of a level vector (training-pair set-up).
 template <typename Tin, typename Tout, bool kToNatural>
 __global__ void k_perm_copy(PermMap pm, int nz, int ny, int nx, const Tin* __restrict__ in, Tout* __restrict__ out)
@@ -1299,22 +1247,9 @@ __device__ __forceinline__ float stencil_at(const ConvGrid& g, const float* __re
     return 26.f * v[p] - off;
 }
 
-// out[p] = (y[p] - y[p + n]) / 2 (natural order).
-__global__ void k_odd_natural(long n, const float* __restrict__ y, float* __restrict__ out)
-{
-    const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if(p < n) out[p] = 0.5f * (y[p] - y[p + n]);
-}
-
-// ------------------------------------------- layers 1 and 3 on the CUDA cores
-// Layer 1 has one real input channel and layer 3 one real output channel, so
-// 15/16 of their tensor-core MMA work multiplies zeros.  For evaluation they
-// run here instead, in FP32 with the BF16-rounded weights: layer 1 fused with
-// the odd pair (the second branch's pre-activation is exactly -z), layer 3
-// fused with the odd combination and the scatter into the level vector.
-
-// Bf16 scalar field of a level: r, or the residual r - A x (k_embed_level's
-// channel 0 without the 15 zero channels and the negated copy).
+// Bf16 scalar field of a level: r (x == nullptr), or the residual r - A x of the
+// 27-point stencil (diagonal diag32, off-diagonals -1), read from colour-permuted
+// level vectors at natural point p.
 __global__ void k_embed_scalar_level(PermMap pm, int nz, int ny, int nx, const float* __restrict__ r,
                                      const float* __restrict__ x, const float* __restrict__ diag32,
                                      __nv_bfloat16* __restrict__ s1)
@@ -1699,8 +1634,8 @@ static int conv_tensor_map(const ConvGrid& g, const void* in, CUtensorMap* map)
 }
 
 template <int kOut>
-static int conv_launch(const ConvGrid& g, const void* in, const void* wB, void* out, const void* act, const PermMap& pm,
-                       int* status, cudaStream_t s)
+static int conv_launch(const ConvGrid& g, const void* in, const void* wB, void* out, const void* act, int* status,
+                       cudaStream_t s)
 {
     static bool attr = false;
     if(!attr)
@@ -1714,23 +1649,19 @@ static int conv_launch(const ConvGrid& g, const void* in, const void* wB, void* 
     const long cap = (long)HB_CONV_CTAS * sm_count();
     const int grid = (int)(tiles < cap ? tiles : cap);
     HB_CUDA(launch_pdl_net(k_conv16<kOut>, dim3(grid), dim3(kConvThreads), (size_t)kConvSmem, s, map, g,
-                           (const __nv_bfloat16*)wB, out, (const __nv_bfloat16*)act, pm, status));
+                           (const __nv_bfloat16*)wB, out, (const __nv_bfloat16*)act, status));
     return 0;
 }
 
 int launch_conv16(const ConvGrid& g, const void* in, const void* wB, int out_mode, void* out, const void* act,
-                  const PermMap* pm, int* status, cudaStream_t s)
+                  int* status, cudaStream_t s)
 {
-    const PermMap none{};
-    const PermMap& m = pm ? *pm : none;
     switch(out_mode)
     {
-        case kOutReluBf16: return conv_launch<kOutReluBf16>(g, in, wB, out, act, m, status, s);
-        case kOutMaskBf16: return conv_launch<kOutMaskBf16>(g, in, wB, out, act, m, status, s);
-        case kOutF32: return conv_launch<kOutF32>(g, in, wB, out, act, m, status, s);
-        case kOutF32C0: return conv_launch<kOutF32C0>(g, in, wB, out, act, m, status, s);
-        case kOutPermSet: return conv_launch<kOutPermSet>(g, in, wB, out, act, m, status, s);
-        case kOutPermAdd: return conv_launch<kOutPermAdd>(g, in, wB, out, act, m, status, s);
+        case kOutReluBf16: return conv_launch<kOutReluBf16>(g, in, wB, out, act, status, s);
+        case kOutMaskBf16: return conv_launch<kOutMaskBf16>(g, in, wB, out, act, status, s);
+        case kOutF32: return conv_launch<kOutF32>(g, in, wB, out, act, status, s);
+        case kOutF32C0: return conv_launch<kOutF32C0>(g, in, wB, out, act, status, s);
         default: return record_error(HPCGB200_ERR_ARG, "conv16: unknown output mode %d", out_mode);
     }
 }
@@ -1809,25 +1740,6 @@ int launch_prepare_weights(const float* w, void* wB, int flip, cudaStream_t s)
     return 0;
 }
 
-int launch_embed_level(const PermMap& pm, int nz, int ny, int nx, const float* r, const float* x,
-                       const float* diag32, void* a, int pair, cudaStream_t s)
-{
-    const long n = (long)nz * ny * nx;
-    k_embed_level<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(pm, nz, ny, nx, r, x, diag32, (__nv_bfloat16*)a,
-                                                              pair);
-    HB_LAUNCHED();
-    return 0;
-}
-
-int launch_odd_combine(const PermMap& pm, int nz, int ny, int nx, const float* y, float* x, bool add, cudaStream_t s)
-{
-    const long n = (long)nz * ny * nx;
-    if(add) k_odd_combine<true><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(pm, nz, ny, nx, y, x);
-    else k_odd_combine<false><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(pm, nz, ny, nx, y, x);
-    HB_LAUNCHED();
-    return 0;
-}
-
 int launch_embed_scalar_level(const PermMap& pm, int nz, int ny, int nx, const float* r, const float* x,
                               const float* diag32, void* s1, cudaStream_t s)
 {
@@ -1872,13 +1784,6 @@ int launch_layer3_grad(const ConvGrid& g, const float* gy, const float* w3, cons
 {
     return pair ? layer1_launch<float, true, true>(g, gy, w3, out, a2, status, s)
                 : layer1_launch<float, false, true>(g, gy, w3, out, a2, status, s);
-}
-
-int launch_odd_natural(long n, const float* y, float* out, cudaStream_t s)
-{
-    k_odd_natural<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, y, out);
-    HB_LAUNCHED();
-    return 0;
 }
 
 int launch_sample_norm(const ConvGrid& g, const float* e, int kind, float* out, cudaStream_t s)
@@ -2000,7 +1905,7 @@ extern "C" int hpcgb200_conv16(int nb, int nz, int ny, int nx, const void* in, c
                      (reinterpret_cast<uintptr_t>(out) & 15) == 0 && (reinterpret_cast<uintptr_t>(act) & 15) == 0,
                  "tensors must be 16-byte aligned");
     const ConvGrid g{nb, nz, ny, nx};
-    return launch_conv16(g, in, wB, out_mode, out, act, nullptr, status, as_stream(stream));
+    return launch_conv16(g, in, wB, out_mode, out, act, status, as_stream(stream));
 }
 
 extern "C" size_t hpcgb200_conv_wgrad_partial_bytes(int nb, int nz, int ny, int nx)

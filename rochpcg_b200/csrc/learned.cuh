@@ -20,8 +20,6 @@ enum ConvOut : int
     kOutMaskBf16 = 1,  // out = bf16(act > 0 ? v : 0), 16 channels (ReLU backward)
     kOutF32 = 2,       // out = v, FP32 16 channels
     kOutF32C0 = 3,     // out = v[0], FP32 scalar field
-    kOutPermSet = 4,   // x[row(p)] = v[0] on a stencil level's colour-permuted vector
-    kOutPermAdd = 5,   // x[row(p)] += v[0]
 };
 
 // Natural grid point -> colour-permuted row of a parity-coloured level.
@@ -45,13 +43,13 @@ struct ConvGrid
 int launch_prepare_weights(const float* w, void* wB, int flip, cudaStream_t s);
 
 // out = conv(in, W) with the epilogue `out_mode`; `act` is the activation
-// tensor of kOutMaskBf16, `pm` the row map of the permuted modes (nb == 1).
+// tensor of kOutMaskBf16.
 int launch_conv16(const ConvGrid& g, const void* in, const void* wB, int out_mode, void* out, const void* act,
-                  const PermMap* pm, int* status, cudaStream_t s);
+                  int* status, cudaStream_t s);
 
-// Evaluation-only kernels: the scalar input field of a level, and the
-// tensor-core forms of the layers with one channel on one side (layer 1: one
-// input channel, layer 3: one output channel).
+// The scalar input field of a level, and the tensor-core forms of the layers
+// with one channel on one side (layer 1: one input channel, layer 3: one output
+// channel).
 // s1 = bf16 scalar field of a level (r, or r - A x when x is not null).
 int launch_embed_scalar_level(const PermMap& pm, int nz, int ny, int nx, const float* r, const float* x,
                               const float* diag32, void* s1, cudaStream_t s);
@@ -78,18 +76,10 @@ int conv16_wgrad_parts(long points);
 int launch_conv16_wgrad(const ConvGrid& g, const void* x, const void* gr, float* partial, float* dw, int* status,
                         cudaStream_t s);
 
-// BF16 16-channel tensor whose channel 0 is a scalar field (others zero):
-// from colour-permuted FP32 level vectors (r, or the residual r - A x when x
-// is not null), or from an FP32 natural field.
-// pair != 0 also writes the negated field as a second sample right after the
-// first (the odd evaluation N(v) - N(-v) as one batch of two).
-int launch_embed_level(const PermMap& pm, int nz, int ny, int nx, const float* r, const float* x,
-                       const float* diag32, void* a, int pair, cudaStream_t s);
+// BF16 16-channel tensor whose channel 0 is an FP32 natural field (others
+// zero).  pair != 0 also writes the negated field as a second sample right after
+// the first (the odd evaluation N(v) - N(-v) as one batch of two).
 int launch_embed_f32(long n, const float* r, void* a, int pair, cudaStream_t s);
-// x[row(p)] = (or +=) (y[p] - y[p + n]) / 2.
-int launch_odd_combine(const PermMap& pm, int nz, int ny, int nx, const float* y, float* x, bool add, cudaStream_t s);
-// out[p] = (y[p] - y[p + n]) / 2.
-int launch_odd_natural(long n, const float* y, float* out, cudaStream_t s);
 // out[b] = 1 / (e_b . e_b) (kind 0) or 1 / (e_b . A e_b) (kind 1, 27-point stencil).
 int launch_sample_norm(const ConvGrid& g, const float* e, int kind, float* out, cudaStream_t s);
 
