@@ -27,8 +27,8 @@ Smoother::Smoother()
     cudaStream_t s = rt().stream;
     w = dalloc<float>(kNetWeights);
     HB_HOST_CUDA(cudaMemsetAsync(w, 0, sizeof(float) * kNetWeights, s));
-    wB = dalloc<unsigned char>(3 * (size_t)hb::kNetWeightTileBytes);
-    wT = dalloc<unsigned char>(3 * (size_t)hb::kNetWeightTileBytes);
+    wB = dalloc<unsigned char>(hb::kNetWeightTileBytes);
+    wT = dalloc<unsigned char>(hb::kNetWeightTileBytes);
     status = dalloc<int>(1);
     HB_HOST_CUDA(cudaMemsetAsync(status, 0, sizeof(int), s));
     HB_HOST_CUDA(cudaStreamSynchronize(s));
@@ -123,18 +123,14 @@ void smoother_set_weights(Smoother& S, const float* host_w, cudaStream_t s)
 int smoother_prepare(Smoother& S, cudaStream_t s)
 {
     if(!S.tiles_stale) return 0;
-    for(int l = 0; l < 3; ++l)
-    {
-        const float* wl = S.w + l * hb::kNetLayerWeights;
-        HB_RETURN_IF(hb::launch_prepare_weights(wl, S.wB + l * hb::kNetWeightTileBytes, 0, s));
-        HB_RETURN_IF(hb::launch_prepare_weights(wl, S.wT + l * hb::kNetWeightTileBytes, 1, s));
-    }
+    const float* w2 = S.w + hb::kNetLayerWeights;
+    // the evaluation's tiles first: its convolution reads them before it waits for
+    // the launch in front of it, and the second launch lies between
+    HB_RETURN_IF(hb::launch_prepare_weights(w2, S.wB, 0, s));
+    HB_RETURN_IF(hb::launch_prepare_weights(w2, S.wT, 1, s));
     S.tiles_stale = false;
     return 0;
 }
-
-static const void* tiles(const Smoother& S, int layer) { return S.wB + layer * hb::kNetWeightTileBytes; }
-static const void* tiles_t(const Smoother& S, int layer) { return S.wT + layer * hb::kNetWeightTileBytes; }
 
 int smoother_level_apply(Smoother& S, const LevelOpt& o, const float* r, float* x, bool residual, cudaStream_t s)
 {
@@ -149,7 +145,7 @@ int smoother_level_apply(Smoother& S, const LevelOpt& o, const float* r, float* 
     const hb::ConvGrid g1{1, L.nz, L.ny, L.nx};
     HB_RETURN_IF(hb::launch_embed_scalar_level(o.pm, L.nz, L.ny, L.nx, r, residual ? x : nullptr, o.diag32, S.a0, s));
     HB_RETURN_IF(hb::launch_layer1_tc(g1, S.a0, 0, S.w, S.a1, S.odd ? 1 : 0, S.status, s));
-    HB_RETURN_IF(hb::launch_conv16(g, S.a1, tiles(S, 1), hb::kOutReluBf16, S.a2, nullptr, S.status, s));
+    HB_RETURN_IF(hb::launch_conv16(g, S.a1, S.wB, hb::kOutReluBf16, S.a2, nullptr, S.status, s));
     return hb::launch_layer3_tc(g1, &o.pm, S.a2, S.w + 2 * hb::kNetLayerWeights, S.odd ? 1 : 0, residual ? 1 : 0, x,
                                 S.status, s);
 }
@@ -161,7 +157,7 @@ int smoother_forward(Smoother& S, const hb::ConvGrid& g, const float* r, float* 
     HB_RETURN_IF(smoother_prepare(S, s));
     const hb::ConvGrid gg{S.odd ? 2 * g.nb : g.nb, g.nz, g.ny, g.nx};
     HB_RETURN_IF(hb::launch_layer1_tc(g, r, 1, S.w, S.a1, S.odd ? 1 : 0, S.status, s));
-    HB_RETURN_IF(hb::launch_conv16(gg, S.a1, tiles(S, 1), hb::kOutReluBf16, S.a2, nullptr, S.status, s));
+    HB_RETURN_IF(hb::launch_conv16(gg, S.a1, S.wB, hb::kOutReluBf16, S.a2, nullptr, S.status, s));
     return hb::launch_layer3_tc(g, nullptr, S.a2, S.w + 2 * hb::kNetLayerWeights, S.odd ? 1 : 0, 2, y, S.status, s);
 }
 
@@ -182,7 +178,7 @@ int smoother_loss_grad(Smoother& S, const hb::ConvGrid& g0, const float* r, cons
     HB_RETURN_IF(hb::launch_layer3_grad(g0, S.y, S.w + 2 * hb::kNetLayerWeights, S.a2, S.d, S.odd ? 1 : 0, S.status, s));
     // layer 2
     HB_RETURN_IF(hb::launch_conv16_wgrad(g, S.a1, S.d, S.partial, dw2, S.status, s));
-    HB_RETURN_IF(hb::launch_conv16(g, S.d, tiles_t(S, 1), hb::kOutMaskBf16, S.g, S.a1, S.status, s));
+    HB_RETURN_IF(hb::launch_conv16(g, S.d, S.wT, hb::kOutMaskBf16, S.g, S.a1, S.status, s));
     // layer 1 (input a0)
     return hb::launch_conv16_wgrad(g, S.a0, S.g, S.partial, dw1, S.status, s);
 }

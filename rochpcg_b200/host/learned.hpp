@@ -11,8 +11,8 @@ constexpr int kNetWeights = 3 * hb::kNetLayerWeights;  // layers 1..3 back to ba
 struct Smoother
 {
     float* w = nullptr;            // FP32 master weights (device)
-    unsigned char* wB = nullptr;   // 3 forward BF16 operand tile sets
-    unsigned char* wT = nullptr;   // 3 transposed-convolution tile sets
+    unsigned char* wB = nullptr;   // layer 2's BF16 operand tiles (layers 1 and 3 read w)
+    unsigned char* wT = nullptr;   // and its transposed convolution's
     bool tiles_stale = true;
     bool odd = false;              // evaluate (N(r) - N(-r)) / 2 (two branches as one batch)
     bool tied = false;             // keep the weights in the tied odd form (one evaluation is odd)
