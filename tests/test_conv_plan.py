@@ -4,8 +4,9 @@ MMAs per (staged plane, row shift) with the dz and dx taps stacked in N, their
 accumulate flags, the shared-memory and TMEM ranges they touch, and the
 epilogue's combination of the dx blocks of neighbouring rows -- checked
 exhaustively for brick depths 1-5 and numerically against a direct 3x3x3
-convolution of one brick.  k_layer3_tc: taps stacked in N, the odd pair folded
-into K, the 27-term gather.  k_layer1_tc: the im2col layout and product."""
+convolution of one brick.  k_layer3_tc: the same plan with one output channel
+and the odd pair folded into K.  k_layer1_tc: the shifted runs and the product.
+k_conv16_wgrad: one unit's MMAs and the sums over its lines."""
 import numpy as np
 import pytest
 
@@ -97,83 +98,140 @@ def test_plan_and_epilogue_equal_a_direct_convolution(ktz):
         assert np.allclose(got, want, rtol=1e-12, atol=1e-12)
 
 
-# ---- the one-channel layers (k_layer3_tc, k_layer1_tc)
+# ---- layer 3 (k_layer3_tc): the same plan with one output channel
 
-K3X, K3Y, K3Z = 16, 8, 2                     # layer-3 output brick
-K3HX, K3HY, K3HZ = K3X + 2, K3Y + 2, K3Z + 2  # its staged box, 720 points
-K3N = 32                                      # 27 taps + 5 zero columns
+P3 = 16  # columns of one output plane: three dx taps, the others zero
 
 
-def test_layer3_tap_stacking_and_pair_folding_equal_the_odd_conv():
-    """D[p][t] = sum_c a[p][c] w[t][c] over the staged points (pair folded into
-    K with the weights halved and negated), then y[o] = sum_t D[o + off_t][t]
-    in tap order, equals (conv(a+) - conv(a-)) / 2 on the brick's outputs."""
+def test_layer3_plan_and_pair_folding_equal_the_odd_conv():
+    """Weight tile (dy, dz) has its three dx taps in columns 0-2; the second
+    branch multiplies the negated weights, both halved, into the same
+    accumulator, which then holds (conv(a+) - conv(a-)) / 2."""
     rng = np.random.default_rng(3)
-    rows = K3HX * K3HY * K3HZ
-    chunks = (rows + 127) // 128
-    assert chunks * 128 >= rows and chunks * K3N * 2 <= 512          # two accumulators fit TMEM
-    pos = rng.standard_normal((K3HZ, K3HY, K3HX, CH))
-    neg = rng.standard_normal((K3HZ, K3HY, K3HX, CH))
-    w = rng.standard_normal((27, CH))                               # w3[t][ci][0]
-    B = np.zeros((K3N, CH))
-    B[:27] = 0.5 * w
-    D = pos.reshape(rows, CH) @ B.T + neg.reshape(rows, CH) @ (-B).T
-    got = np.zeros((K3Z, K3Y, K3X))
-    for oz in range(K3Z):
-        for oy in range(K3Y):
-            for ox in range(K3X):
-                s = 0.0
-                for t in range(27):
-                    dz, dy, dx = t // 9 - 1, (t // 3) % 3 - 1, t % 3 - 1
-                    r = ((oz + 1 + dz) * K3HY + (oy + 1 + dy)) * K3HX + (ox + 1 + dx)
-                    assert 0 <= r < rows
-                    s += D[r, t]
-                got[oz, oy, ox] = s
-    want = np.zeros((K3Z, K3Y, K3X))
-    for t in range(27):
-        dz, dy, dx = t // 9 - 1, (t // 3) % 3 - 1, t % 3 - 1
-        sl = (slice(1 + dz, 1 + dz + K3Z), slice(1 + dy, 1 + dy + K3Y), slice(1 + dx, 1 + dx + K3X))
-        want += 0.5 * (pos[sl] @ w[t] - neg[sl] @ w[t])
-    assert np.allclose(got, want, rtol=1e-12, atol=1e-12)
+    ktz = 4
+    pos, neg = rng.standard_normal((2, ktz + 2, KHY, KTX, CH))
+    w = rng.standard_normal((27, CH))                                  # w3[t][ci][0]
+    B = np.zeros((9 * P3, CH))                                         # rows (dy, dz = +1, 0, -1, column)
+    for tile in range(9):
+        for col in range(3):
+            B[tile * P3 + col] = 0.5 * w[(2 - tile % 3) * 9 + tile // 3 * 3 + col]
+    D = np.full((128, ktz * P3), np.nan)
+    n = 0
+    for q, dyi, m0, m1, acc in plan(ktz):
+        r0 = (dyi * 3 + m0 - q + 2) * P3
+        nrows = (m1 - m0 + 1) * P3
+        assert nrows in (16, 32, 48) and 0 <= r0 and r0 + nrows <= B.shape[0]
+        cols = slice(m0 * P3, m0 * P3 + nrows)
+        for box, sign, add in ((pos, 1.0, acc), (neg, -1.0, 1)):
+            prod = box[q, dyi:dyi + KTY].reshape(128, CH) @ (sign * B[r0:r0 + nrows]).T
+            D[:, cols] = prod if add == 0 else D[:, cols] + prod
+            n += 1
+    assert n == 42 and 2 * ktz * P3 <= 128                             # two accumulators in 128 columns
+    for mt in range(ktz):
+        blk = D[:, mt * P3:(mt + 1) * P3].reshape(KTY, KTX, P3)
+        got = blk[:, 0:14, 0] + blk[:, 1:15, 1] + blk[:, 2:16, 2]
+        want = np.zeros((KTY, 14))
+        for t in range(27):
+            dz, dy, dx = t // 9 - 1, (t // 3) % 3 - 1, t % 3 - 1
+            sl = (mt + 1 + dz, slice(1 + dy, 1 + dy + KTY), slice(1 + dx, 15 + dx))
+            want += 0.5 * (pos[sl] - neg[sl]) @ w[t]
+        assert np.allclose(got, want, rtol=1e-12, atol=1e-12)
+        assert not blk[..., 3:].any()
+
+
+# ---- layer 1 (k_layer1_tc): taps as K, the operand MN-major
+
+K1_GROUP, K1_PLANE = 32 * 16 + 16, 16 * (32 * 16 + 16)  # bytes of an 8-point group and of a plane
 
 
 def k1_off(r, c8):
-    """Byte offset of im2col row r, 8-element K chunk c8 (k_layer1_tc)."""
+    """Byte offset of weight row r, 8-element K chunk c8."""
     return (r >> 3) * 512 + c8 * 128 + (r & 7) * 16
 
 
-def test_layer1_im2col_layout_tiles_its_plane():
-    """128 rows x 4 K chunks of 16 bytes fill one 8 KB plane exactly once; the
-    MMA's K halves start 256 B apart with LBO 128 and SBO 512; the 16 x 32
-    weight operand ends at 1 KB."""
-    offs = sorted(k1_off(r, c) for r in range(128) for c in range(4))
-    assert offs == list(range(0, 8192, 16))
-    for r in range(128):
+def test_layer1_weight_operand():
+    """The MMA's K halves start 256 B apart with LBO 128 and SBO 512; 16 rows x 32 taps end at 1 KB."""
+    for r in range(16):
         for c in range(4):
             kh, cc = divmod(c, 2)
             assert k1_off(r, c) == kh * 256 + (r >> 3) * 512 + cc * 128 + (r & 7) * 16
     assert max(k1_off(co, t >> 3) + (t & 7) * 2 for co in range(16) for t in range(32)) == 1022
 
 
-def test_layer1_im2col_product_equals_the_conv():
-    """Each row = the 27 neighbours of its point (5 zero taps); the K = 32
-    product with w1[t][0][co] gives layer 1's 16 pre-activations."""
+def test_layer1_runs_make_the_operand_of_the_conv():
+    """A thread's line of ten points is stored as three shifted runs of eight
+    for each (dz, dy) it serves; read as the MMA reads it (8-point groups SBO
+    apart, taps 16 B apart), element (m, t) is the neighbour of point m at tap t."""
     rng = np.random.default_rng(4)
-    hz, hy, hx = 6, 10, 18
-    field = rng.standard_normal((hz, hy, hx))
+    field = rng.standard_normal((6, 10, 18))
     w = rng.standard_normal((27, CH))
-    Bw = np.zeros((32, CH))
-    Bw[:27] = w
-    for q in range(4):
-        A = np.zeros((128, 32))
-        for m in range(128):
-            mx, my = m % 16, m // 16
-            for t in range(27):
-                dz, dy, dx = t // 9 - 1, (t // 3) % 3 - 1, t % 3 - 1
-                A[m, t] = field[q + 1 + dz, my + 1 + dy, mx + 1 + dx]
-        got = (A @ Bw).reshape(8, 16, CH)
+    smem = np.full(4 * K1_PLANE // 2, np.nan)                          # two-byte elements
+    for g in range(4 * 16):                                            # the zero taps
+        at = (g * K1_GROUP + 27 * 16) // 2
+        smem[at:at + 40] = 0.0
+    for line in range(120):
+        half, hy, hz = line & 1, (line >> 1) % 10, (line >> 1) // 10
+        v = field[hz, hy, 8 * half:8 * half + 10]
+        for dz in range(3):
+            for dy in range(3):
+                oz, oy = hz - dz, hy - dy
+                if not (0 <= oz < 4 and 0 <= oy < 8):
+                    continue
+                for dx in range(3):
+                    at = (oz * K1_PLANE + (2 * oy + half) * K1_GROUP + (dz * 9 + dy * 3 + dx) * 16) // 2
+                    assert np.isnan(smem[at:at + 8]).all()             # nobody else's
+                    smem[at:at + 8] = v[dx:dx + 8]
+    for oz in range(4):
+        A = np.array([[smem[(oz * K1_PLANE + kh * 256 + (m >> 3) * K1_GROUP + k * 16) // 2 + (m & 7)]
+                       for kh in range(2) for k in range(16)] for m in range(128)])
+        got = (A[:, :27] @ w).reshape(8, 16, CH)
         want = np.zeros((8, 16, CH))
         for t in range(27):
-            dz, dy, dx = t // 9 - 1, (t // 3) % 3 - 1, t % 3 - 1
-            want += field[q + 1 + dz, 1 + dy:9 + dy, 1 + dx:17 + dx][..., None] * w[t]
+            dz, dy, dx = t // 9, (t // 3) % 3, t % 3
+            want += field[oz + dz, dy:8 + dy, dx:16 + dx][..., None] * w[t]
+        assert not A[:, 27:].any()
         assert np.allclose(got, want, rtol=1e-12, atol=1e-12)
+
+
+# ---- weight gradient (k_conv16_wgrad): plain bricks, a tap is a start address
+
+WX, WLINES, WZ = 16, 3, 8
+ROW_A, ROW_B = (WX + 2) * 8, WX * 8                                    # elements of one line of one 8-channel half
+PLANE_A, PLANE_B = (WLINES + 2) * 2 * ROW_A, WLINES * 2 * ROW_B
+WN = WLINES * CH
+
+
+def test_weight_gradient_unit_equals_the_direct_sums():
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((WZ + 2, WLINES + 2, WX + 2, CH))
+    g = rng.standard_normal((WZ, WLINES, WX, CH))
+    # [plane][line][half][x][8 channels]; the bytes behind the last plane are read, and ignored
+    sa = np.concatenate([x.reshape(WZ + 2, WLINES + 2, WX + 2, 2, 8).transpose(0, 1, 3, 2, 4).ravel(),
+                         g.reshape(WZ, WLINES, WX, 2, 8).transpose(0, 1, 3, 2, 4).ravel()])
+    off_b = (WZ + 2) * PLANE_A
+    k = np.arange(WX)[:, None]
+    m = np.arange(128)[None, :]
+    D = np.full((128, 9 * WN), np.nan)
+    started = set()
+    for i in range(WZ + 2):
+        q = (i + 2) % (WZ + 2)
+        lo, hi = (2 - q if q < 2 else 0), (WZ + 1 - q if q > WZ - 1 else 2)
+        n = np.arange((hi - lo + 1) * WN)[None, :]
+        for t in range(3):
+            a = sa[q * PLANE_A + t * 8 + (m >> 3) * ROW_A + k * 8 + (m & 7)]
+            b = sa[off_b + (q - 2 + lo) * PLANE_B + (n >> 3) * ROW_B + k * 8 + (n & 7)]
+            cols = slice((3 * t + lo) * WN, (3 * t + hi + 1) * WN)
+            if i == 0:
+                assert (lo, hi) == (0, 2)
+                D[:, cols] = a.T @ b
+                started.add(t)
+            else:
+                D[:, cols] += a.T @ b
+    assert started == {0, 1, 2}
+    for t in range(27):
+        dz, dy, dx = t // 9 - 1, (t // 3) % 3 - 1, t % 3 - 1
+        block = 3 * (dx + 1) + 1 - dz
+        got = sum(D[(dy + 1 + r) * CH:(dy + 2 + r) * CH, block * WN + r * CH:block * WN + (r + 1) * CH]
+                  for r in range(WLINES))
+        want = np.einsum("zyxi,zyxo->io", x[1 + dz:1 + dz + WZ, 1 + dy:1 + dy + WLINES, 1 + dx:1 + dx + WX], g)
+        assert np.allclose(got, want, rtol=1e-11, atol=1e-11)
