@@ -1290,8 +1290,8 @@ __device__ __forceinline__ float in_value(const float* v, long q) { return __bfl
 // a 128^3 sample.  Here A is MN-major: eight points along x are the 16 bytes of
 // one tap.  A thread reads ten points of one line of the halo'd brick, rounds
 // them once, and the three shifted runs of eight (dx = -1, 0, +1) are stored for
-// each of the up to nine (dz, dy) the line serves: 27 16-byte stores for 240
-// values.  Tap runs of an 8-point group are contiguous (K core matrices 128 B
+// each of the up to nine (dz, dy) the line serves: 27 16-byte stores, 216 values
+// of the operand from ten points read.  Tap runs of an 8-point group are contiguous (K core matrices 128 B
 // apart), groups 528 B apart, which spreads a store over all banks.  The
 // epilogue writes relu(z) and, for the odd pair, relu(-z) as BF16, a point's 32
 // bytes at a time (in two halves the stores were the bound: the new gather alone
@@ -1496,7 +1496,7 @@ __global__ void k_sample_norm(ConvGrid g, const float* __restrict__ e, int kind,
     if(threadIdx.x == 0) out[blockIdx.x] = (float)(1.0 / s);
 }
 
-// d = y - e, y the network output (odd: (y[p] - y[p + n]) / 2).
+// d = y - e, y the network output, one value a point (odd: already combined).
 __global__ void k_loss_diff(long n, const float* __restrict__ y, const float* __restrict__ e, float* __restrict__ d)
 {
     const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;

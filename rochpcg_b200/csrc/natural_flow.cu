@@ -3,13 +3,14 @@
 //
 // What bounds it: the sweep is a chain of nx + 2 (ny-1) + 4 (nz-1) dependent
 // rows (natural.cuh's fronts), each a chain of 20 FP64 adds and a division;
-// one launch per front takes 5 us a front, this form 0.65 us (104^3, hand-offs
-// between blocks included; 0.34 us within a block of one plane): the 104^3
-// reference V-cycle went from 51.3 to 3.9 ms.  Here a block owns a group of z planes, one thread
-// per grid line along x, and steps along s = ix + 2 iy; plane lz of the group
-// runs four steps behind plane lz - 1, which is the fronts' order, so one
-// __syncthreads per front replaces a launch and new values pass between lines
-// through shared memory.  Groups pipeline: the last plane of a group is read
+// one launch per front takes 11.7 us a front (104^3 step, 1444 launches: 16.8 ms,
+// the host issues them), this form 0.77 us with the check and the re-laying (1.11
+// ms), 0.68 in the sweeps alone, hand-offs between blocks included (0.34 within a
+// block of one plane): the 104^3 reference V-cycle went from 54.8 to 3.9 ms.  Here
+// a block owns a group of z planes, one thread per grid line along x, and steps
+// along s = ix + 2 iy; plane lz of the group runs four steps behind plane lz - 1,
+// which is the fronts' order, so one __syncthreads per front replaces a launch and
+// new values pass between lines through shared memory.  Groups pipeline: the last plane of a group is read
 // by the next group's block from global memory, every value being its own
 // ready flag (the buffer is filled with a NaN pattern no computation returns),
 // so a value costs one L2 round trip and no fence.

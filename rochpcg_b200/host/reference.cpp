@@ -68,8 +68,8 @@ bool capturing(cudaStream_t s)
 // workspace kept beside the generated arrays, or one launch per front where a
 // plane has too many lines for them, the workspace cannot be had, or the
 // stream is being captured (nobody could read the status of a replay's waits).
-// 104^3: 10.3 ms with the 1444 launches of the fronts.  repeated: the previous
-// sweep on this level had the same matrix and r.
+// 104^3: 16.8 ms with the 1444 launches of the fronts, 1.1 ms so.  repeated: the
+// previous sweep on this level had the same matrix and r.
 int symgs_ref(const SparseMatrix& A, const Vector& r, Vector& x, bool repeated)
 {
     const hb::NaturalLevel L = natural(A);
