@@ -150,3 +150,23 @@ def test_cycle_on_changed_ell_arrays(dims, what):
         _launches(P, 0, r, y, False)
         sync(P)
         assert np.array_equal(_mg(P, r, R.MODE_FP64), host(y))
+
+
+def test_solve_on_changed_ell_arrays():
+    """A captured FP64 solve and its V-cycle against the CPU restatement on the same changed arrays."""
+    O = ColoredProblem(32, 32, 32)
+    with R.Problem(32) as P:
+        healthy = P.cg(8, 0.0)["hist"]
+        for level, slot in ((0, 4), (1, 20)):
+            lev = O.levels[level]
+            row = int(np.flatnonzero((lev.ell_col >= 0).all(0))[11])
+            lev.ell_val[slot, row] = -0.5
+            lev.ell_col[4, row] += 1  # the neighbouring row of the same colour
+            for f, a in (("ell_val", lev.ell_val), ("ell_col", lev.ell_col)):
+                dev_field(P, f, level, a.dtype).copy_(torch.from_numpy(a.ravel()))
+        torch.cuda.synchronize()
+        r = np.random.default_rng(9).normal(size=O.levels[0].m)
+        assert np.array_equal(_mg(P, to_dev(r), R.MODE_FP64), O.mg(r))
+        got, want = P.cg(8, 0.0)["hist"], O.cg(8, 0.0)["hist"]
+        # dot products in another order, as on the healthy matrix
+        assert np.allclose(got, want, rtol=1e-8, atol=0) and not np.allclose(got, healthy, rtol=1e-6, atol=0)
